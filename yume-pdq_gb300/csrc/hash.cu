@@ -37,6 +37,7 @@
 namespace ypdq {
 
 __device__ float g_dct[16 * 127];  // D[k][i] = sqrt(2/127) cos(pi (k+1) (2i+1) / 254), f32
+__device__ alignas(16) float g_dct_t[128 * 16];  // the same as D^T: [i][k]; row 127 is zero
 
 constexpr int kStagesPerImage = 128;  // stage s holds rows 4s+1 .. 4s+4 (stage 127: 509, 510)
 constexpr int kComputeThreads = 128;
@@ -159,6 +160,32 @@ struct CompressIn<Tin, true> {
   using T = float;
 };
 
+// Two f32 operations in one instruction, each rounded by itself. ptxas (13.0) contracts a
+// packed multiply and the packed add that takes its result into one fused operation, .rn or
+// not (scalar mul.rn / add.rn it leaves alone), which would change bits. So a product is
+// taken as fma(a, b, -0) with the -0 read from the launch parameters, a value that the
+// compiler does not know: RN(a b + -0) is RN(a b), signed zeros included, and an fma cannot
+// be contracted with a later add.
+__device__ __forceinline__ float2 fma2_rn(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mov.b64 w, {%6, %7};\n\tfma.rn.f32x2 z, x, y, w;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b, float neg_zero) {
+  return fma2_rn(a, b, make_float2(neg_zero, neg_zero));
+}
+__device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
 // ITU-R BT.601 luma in the reference's scalar order (Kernel::cvt_rgb8_to_luma8f,
 // src/kernel/mod.rs:303-340, coefficients src/kernel/constants.rs:23):
 // (0.299 r + 0.587 g) + 0.114 b, each product and sum rounded to f32, no fused multiply-add.
@@ -227,6 +254,28 @@ __device__ __forceinline__ void load_row8(const uint8_t* row, int j, float x[8])
   uint32_t a = r[j], b = r[j + 1];
   x[0] = byte_f<0>(a); x[1] = byte_f<1>(a); x[2] = byte_f<2>(a); x[3] = byte_f<3>(a);
   x[4] = byte_f<0>(b); x[5] = byte_f<1>(b); x[6] = byte_f<2>(b); x[7] = byte_f<3>(b);
+}
+
+// RGB columns as f32 luma, converted on load (hash_split_kernel; hash_kernel converts whole
+// stages once instead, see convert_stage_warp).
+__device__ __forceinline__ void load_row8(const rgb8_t* row, int j, float x[8]) {
+  const uint32_t* r = reinterpret_cast<const uint32_t*>(row) + 3 * j;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {  // 12 bytes each: r g b r | g b r g | b r g b
+    const uint32_t a = r[3 * h], b = r[3 * h + 1], c = r[3 * h + 2];
+    x[4 * h + 0] = luma_bt601(byte_f<0>(a), byte_f<1>(a), byte_f<2>(a));
+    x[4 * h + 1] = luma_bt601(byte_f<3>(a), byte_f<0>(b), byte_f<1>(b));
+    x[4 * h + 2] = luma_bt601(byte_f<2>(b), byte_f<3>(b), byte_f<0>(c));
+    x[4 * h + 3] = luma_bt601(byte_f<1>(c), byte_f<2>(c), byte_f<3>(c));
+  }
+}
+__device__ __forceinline__ void load_row8(const rgba8_t* row, int j, float x[8]) {
+  const uint4* r = reinterpret_cast<const uint4*>(row);
+  const uint4 a = r[j], b = r[j + 1];
+  const uint32_t px[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    x[k] = luma_bt601(byte_f<0>(px[k]), byte_f<1>(px[k]), byte_f<2>(px[k]));
 }
 
 #define YPDQ_W(di, dj) __uint_as_float(YPDQ_TENT_BITS_##di##_##dj)
@@ -986,6 +1035,385 @@ fail:
   }
 }
 
+// --------------------------------------------------------------- split kernel
+//
+// hash_split_kernel: the FP32 hash of a small batch, one image per cluster of 8 CTAs.
+//
+// hash_kernel walks an image's 128 stages one after another on one CTA, ~40 us whatever the
+// batch, so a batch of fewer images than CTAs leaves most of the chip idle and waits for a
+// latency chain. Here the image is cut by rows: CTA c of the cluster copies the 66 input
+// rows of compressed rows 16 c .. 16 c + 15 at once (five bulk copies, no ring), and the
+// chains that are serial by definition are cut along their independent directions:
+//   compress  CTA c, thread (column j, group g): rows 16 c + 4 g .. + 3 of column j, each
+//             value sent to the CTA that owns column j (16 columns per CTA) by an
+//             asynchronous store into its shared memory;
+//   stage 1   CTA c: T[k][j] of its 16 columns, the reference's four partial sums over i in
+//             four lanes, each 32 steps long; T goes to the cluster's first CTA;
+//   stage 2   first CTA: P[k][c], the same routine with T in the place of the image;
+//   epilogue  first CTA: four warps select one median each and pack its two slots; eight
+//             warps sum one slot's gradients (480 dependent additions, the longest chain).
+// Every sum keeps its order, so the results are hash_kernel's bit for bit.
+//
+// Bound by the latency of that sequence: of ~12,500 clk for one f32 image, ~2,800 until the
+// rows are there, ~2,000 compress (8 conflict-free 16-byte loads per value), ~500 for each of
+// the two exchanges, ~1,150 per DCT stage and ~4,200 epilogue (2,150 of them the gradient
+// sum). Back to back, one image: 8.5 us (hash_kernel 40.6; RGB8 10.4, was 77); 37 u8 images
+// 14.6 us (43.2); 64 f32 images 32 us (41.3).
+constexpr int kSplitCtas = 8;        // CTAs per image (the portable cluster size)
+constexpr int kSplitThreads = 512;
+constexpr int kSplitRows = 128 / kSplitCtas;           // compressed rows per CTA
+constexpr int kSplitInRows = 4 * kSplitRows + 2;       // input rows they read
+constexpr int kSplitCopies = (kSplitInRows + 15) / 16; // bulk copies of up to 16 rows
+
+constexpr int kSplitPitch = 132;  // floats per column of a stage's input (16-byte columns)
+
+struct SplitSmem {
+  // stage inputs column by column: the lanes of the four partial sums read values
+  // 4 s .. 4 s + 3 of 8 columns, 32 different banks at this pitch.
+  // [0]: compressed columns 16 c .. 16 c + 15; [1], first CTA only: T[k][j]
+  alignas(16) float in[2][16][kSplitPitch];
+  alignas(16) float dt[128][16];   // dt[i][k] = D[k][i]; row 127 is zero
+  float p[16][17];                 // PDQF, padded: slots 4-7 read it by columns
+  alignas(16) float grad[8][500];  // |differences| of a slot in summation order, padded
+  uint64_t full[kSplitCopies];     // input rows
+  uint64_t dt_full, in_full[2];    // DCT matrix; stage inputs, from all CTAs
+  int abort_flag;
+};
+constexpr int kSplitRowsOffset = (sizeof(SplitSmem) + 127) & ~127;  // the input rows follow
+
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// Address of `p` (a place in this CTA's shared memory) in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_cluster(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ uint64_t policy_evict_last() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+// Asynchronous stores to another CTA that count their bytes on its mbarrier: the receiver
+// waits for the data alone (one way), where a cluster barrier after plain stores waits for
+// their acknowledgement and then for the barrier (~1,300 clk measured).
+__device__ __forceinline__ void st_async4(uint32_t dst, uint32_t bar, float x, float y, float z,
+                                          float w) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+      ::"r"(dst), "r"(__float_as_uint(x)), "r"(__float_as_uint(y)), "r"(__float_as_uint(z)),
+      "r"(__float_as_uint(w)), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void st_async1(uint32_t dst, uint32_t bar, float x) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
+               "r"(__float_as_uint(x)), "r"(bar)
+               : "memory");
+}
+
+// One DCT stage of 16 x 16 outputs by 128 threads: out(x, y) = sum over m < 127 of
+// in[stage][x][m] * D[y][m] in the reference's four partial sums. Thread (warp w, lane):
+// partial sum r = lane / 8, x = lane % 8 and x + 8, y = 4 w .. + 3 (the D values serve two
+// columns: the loads, four wavefronts for four D values, are what bounds this loop); the
+// sums are combined in lanes 0-7. Stage 0 (stage 1 of the DCT) sends T[y][16 rank + x] to
+// the first CTA, stage 1 writes P[x][y].
+// (Row 127 of the input and of D^T is zero: it adds +-0 to a sum that is never -0.)
+__device__ __forceinline__ void split_dct_stage(SplitSmem& sm, int stage, int rank, int w,
+                                                int lane, float neg_zero) {
+  const int r = lane >> 3, x = lane & 7, y0 = 4 * w;
+  const float* src = &sm.in[stage][x][r];
+  const float* dsrc = &sm.dt[r][y0];
+  float2 a[2][2] = {};  // [column][pair of y]
+#pragma unroll 8
+  for (int s = 0; s < 32; ++s) {  // m = 4 s + r
+    const float b0 = src[4 * s], b1 = src[4 * s + 8 * kSplitPitch];
+    const float4 d = *reinterpret_cast<const float4*>(dsrc + 64 * s);
+    const float2 d0 = make_float2(d.x, d.y), d1 = make_float2(d.z, d.w);
+    a[0][0] = add2_rn(a[0][0], mul2_rn(d0, make_float2(b0, b0), neg_zero));
+    a[0][1] = add2_rn(a[0][1], mul2_rn(d1, make_float2(b0, b0), neg_zero));
+    a[1][0] = add2_rn(a[1][0], mul2_rn(d0, make_float2(b1, b1), neg_zero));
+    a[1][1] = add2_rn(a[1][1], mul2_rn(d1, make_float2(b1, b1), neg_zero));
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float v[4] = {a[h][0].x, a[h][0].y, a[h][1].x, a[h][1].y};
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      const float s1 = __shfl_down_sync(0xffffffffu, v[y], 8);
+      const float s2 = __shfl_down_sync(0xffffffffu, v[y], 16);
+      const float s3 = __shfl_down_sync(0xffffffffu, v[y], 24);
+      v[y] = __fadd_rn(__fadd_rn(__fadd_rn(v[y], s1), s2), s3);
+    }
+    if (lane < 8) {
+      if (stage == 0) {
+        const uint32_t bar = map_cluster(&sm.in_full[1], 0);
+        const uint32_t dst = map_cluster(&sm.in[1][y0][16 * rank + x + 8 * h], 0);
+#pragma unroll
+        for (int y = 0; y < 4; ++y) st_async1(dst + 4 * kSplitPitch * y, bar, v[y]);
+      } else {
+#pragma unroll
+        for (int y = 0; y < 4; ++y) sm.p[x + 8 * h][y0 + y] = v[y];
+      }
+    }
+  }
+}
+
+// The rank-127 value of 256 held 8 per lane: MSB-first radix selection like
+// select_rank127_x4's, three bits at a time: each lane counts its keys per digit in eight
+// 4-bit counters (at most 8 each), which are widened to 16 bits and summed over the warp by
+// four independent reductions. Once the digit's bin holds one key, that key is the answer
+// (after 4 or 5 of the 11 rounds on images).
+__device__ __forceinline__ float select_rank127(const float (&v)[8]) {
+  uint32_t key[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) key[e] = f32_key(v[e]);
+  uint32_t prefix = 0u;
+  int rank = 127;
+#pragma unroll 1
+  for (int shift = 29;; shift = shift > 3 ? shift - 3 : 0) {
+    uint32_t counts = 0u;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const uint32_t k = (key[e] ^ prefix) >> shift;  // above 7: another prefix
+      counts += k < 8u ? 1u << (4 * k) : 0u;
+    }
+    // (in the last round, shift 0 with two bits left, digits 4-7 are keys of another prefix;
+    // the rank lies below them)
+    uint32_t two[4];  // digits i and i + 4 in 16-bit halves
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      two[i] = __reduce_add_sync(0xffffffffu, (counts >> (4 * i)) & 0x000F000Fu);
+    int below = 0, upto = 256, digit = 0, cum = 0;  // keys below and up to the rank's digit
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+      cum += static_cast<int>((d & 4) ? two[d & 3] >> 16 : two[d & 3] & 0xFFFFu);
+      if (cum <= rank) {
+        below = cum;
+        digit = d + 1;
+      } else {
+        upto = min(upto, cum);
+      }
+    }
+    prefix |= static_cast<uint32_t>(digit) << shift;
+    if (shift == 0) return key_f32(prefix);
+    if (upto - below == 1) {
+      uint32_t found = 0u;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) found |= ((key[e] ^ prefix) >> shift) == 0u ? key[e] : 0u;
+      return key_f32(__reduce_or_sync(0xffffffffu, found));
+    }
+    rank -= below;
+  }
+}
+
+// Slot s as signs and strides over P (pitch 17): value (r, c) is P[r row + c col] with its sign bit
+// flipped where bit r of `rows` and bit c of `cols` differ (see slot_rows).
+struct SlotView {
+  const float* P;
+  int row, col;
+  uint32_t rows, cols;
+  __device__ __forceinline__ SlotView(const float* P_, int s, uint32_t rm, uint32_t cm)
+      : P(P_), row(s < 4 ? 17 : 1), col(s < 4 ? 1 : 17), rows(slot_rows(s) ? rm : 0u),
+        cols(slot_cols(s) ? cm : 0u) {}
+  __device__ __forceinline__ float at(int r, int c) const {
+    return __uint_as_float(__float_as_uint(P[r * row + c * col]) ^
+                           (((rows >> r) ^ (cols >> c)) << 31));
+  }
+};
+
+// Quality of slot s by one warp: its 480 absolute differences in parallel into `g` in the
+// reference's order (240 down the columns, row by row, then 240 along the rows), then the
+// sequential sum in lane 0 (480 dependent additions, the loads 16 values ahead of them).
+// Of |s x - s' y| with signs s and s' only their product matters.
+__device__ __forceinline__ void split_quality(const float* P, int s, uint32_t rm, uint32_t cm,
+                                              int lane, float* g, float* quality) {
+  const SlotView m(P, s, rm, cm);
+  const int r0 = lane >> 4, c = lane & 15;
+  const float* p = P + r0 * m.row + c * m.col;
+  const int right = c < 15 ? m.col : 0;
+  // bit 2 t: rows r0 + 2 t and r0 + 2 t + 1 differ in sign; all bits: columns c and c + 1 do
+  const uint32_t rdiff = (m.rows ^ (m.rows >> 1)) >> r0;
+  const uint32_t cdiff = ((m.cols ^ (m.cols >> 1)) >> c) << 31;
+#pragma unroll
+  for (int t = 0; t < 8; ++t, p += 2 * m.row) {
+    // (the last row's lower neighbour is past the matrix, inside the shared struct: unused)
+    const float x = p[0];
+    const float below = __uint_as_float(__float_as_uint(p[m.row]) ^ ((rdiff >> (2 * t)) << 31));
+    const float beside = __uint_as_float(__float_as_uint(p[right]) ^ cdiff);
+    if (t < 7 || r0 == 0) g[16 * (r0 + 2 * t) + c] = fabsf(__fsub_rn(x, below));
+    if (c < 15) g[240 + 15 * (r0 + 2 * t) + c] = fabsf(__fsub_rn(x, beside));
+  }
+  __syncwarp();
+  if (lane != 0) return;
+  const float4* g4 = reinterpret_cast<const float4*>(g);
+  float4 a[4], b[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) a[q] = g4[q];
+  float sum = 0.0f;
+#pragma unroll 1
+  for (int t = 0; t < 120; t += 8) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) b[q] = g4[t + 4 + q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, a[q].x), a[q].y), a[q].z), a[q].w);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] = g4[t + 8 + q];  // the last step reads the padding
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, b[q].x), b[q].y), b[q].z), b[q].w);
+  }
+  quality[s] = fminf(__fdiv_rn(sum, 180.0f), 1.0f);
+}
+
+// Median, bits and outputs of slots s and s + 4 (s < 4; slot s + 4 is slot s's transpose
+// with the other axis' signs, at slot s's threshold) by one warp.
+__device__ __forceinline__ void split_slots(const float* P, int s, uint32_t rm, uint32_t cm,
+                                            int lane, const EpilogueOut& o) {
+  const int i = lane >> 1, j0 = (lane & 1) << 3;
+  float v[2][8];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const SlotView m(P, s + 4 * h, rm, cm);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[h][e] = m.at(i, j0 + e);
+  }
+  const float thr = select_rank127(v[0]);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int slot = s + 4 * h;
+    uint32_t byte = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) byte |= (v[h][e] > thr ? 1u : 0u) << e;
+    if (o.hashes) o.hashes[slot * 32 + 31 - lane] = static_cast<uint8_t>(byte);
+    if (o.pdqf && (slot == 0 || o.pdqf_slots == 8)) {
+      float4* dst = reinterpret_cast<float4*>(o.pdqf + slot * 256 + lane * 8);
+      dst[0] = make_float4(v[h][0], v[h][1], v[h][2], v[h][3]);
+      dst[1] = make_float4(v[h][4], v[h][5], v[h][6], v[h][7]);
+    }
+    if (o.thresholds && lane == 0) o.thresholds[slot] = thr;
+  }
+}
+
+template <typename Tin>
+__global__ void __cluster_dims__(kSplitCtas, 1, 1) __launch_bounds__(kSplitThreads, 2)
+    hash_split_kernel(const HashLaunch prm) {
+  constexpr int kRowBytes = InputTraits<Tin>::kRowBytes;
+  extern __shared__ unsigned char smem_raw[];
+  SplitSmem& sm =
+      *reinterpret_cast<SplitSmem*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
+  unsigned char* const rows = reinterpret_cast<unsigned char*>(&sm) + kSplitRowsOffset;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = static_cast<int>(cluster_ctarank());
+  const int64_t n = blockIdx.x / kSplitCtas;
+  if (prm.n_dev && n >= *prm.n_dev) return;  // the whole cluster
+  const int row0 = 4 * kSplitRows * rank + 1;  // first input row
+  if (tid < kSplitCopies) {  // one lane per copy
+    mbar_init(&sm.full[tid], 1);
+    fence_mbar_init();
+    const unsigned char* img =
+        static_cast<const unsigned char*>(prm.images) + n * (512ll * kRowBytes);
+    // rows past 510 are read by no output
+    const int first = row0 + 16 * tid;
+    const int count = min(min(16, kSplitInRows - 16 * tid), 511 - first);
+    if (count > 0) {
+      const uint32_t bytes = static_cast<uint32_t>(count) * kRowBytes;
+      mbar_arrive_expect_tx(&sm.full[tid], bytes);
+      bulk_g2s(rows + 16 * tid * kRowBytes, img + static_cast<int64_t>(first) * kRowBytes, bytes,
+               &sm.full[tid], policy_evict_first());
+    }
+  } else if (tid == 32) {
+    mbar_init(&sm.dt_full, 1);
+    mbar_init(&sm.in_full[0], 1);
+    mbar_init(&sm.in_full[1], 1);
+    sm.abort_flag = 0;
+    fence_mbar_init();
+    mbar_arrive_expect_tx(&sm.in_full[0], 16 * 128 * 4);
+    if (rank == 0) mbar_arrive_expect_tx(&sm.in_full[1], 16 * 128 * 4);
+    mbar_arrive_expect_tx(&sm.dt_full, sizeof(sm.dt));
+    bulk_g2s(sm.dt, g_dct_t, sizeof(sm.dt), &sm.dt_full, policy_evict_last());
+  }
+  __syncthreads();
+  cluster_arrive();  // this CTA runs and its barriers are set: the others may write to it
+
+  // ---- compress: thread (j, g), rows 4 g .. 4 g + 3 of the CTA's 16
+  const int j = tid & 127, g = tid >> 7;
+  volatile int* abort_flag = &sm.abort_flag;
+  bool ok = mbar_wait(&sm.full[g], 0, abort_flag);
+  // the last output's last two input rows are in the next copy (none past the image's end)
+  if (row0 + 16 * (g + 1) <= 510) ok &= mbar_wait(&sm.full[g + 1], 0, abort_flag);
+  float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  const int i0 = kSplitRows * rank + 4 * g;
+  if (j < 127) {
+    CompressCarry cc{};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (i0 + r < 127) {
+        const Tin* st = reinterpret_cast<const Tin*>(rows + (4 * (4 * g + r)) * kRowBytes);
+        b[r] = compress_next<Tin>(st, st + 4 * 512, j, r == 0, cc);
+        if (prm.buf1) prm.buf1[(n * 127 + i0 + r) * 128 + j] = b[r];
+      }
+    }
+  }
+  cluster_wait();
+  {
+    const uint32_t owner = static_cast<uint32_t>(j >> 4);
+    st_async4(map_cluster(&sm.in[0][j & 15][i0], owner), map_cluster(&sm.in_full[0], owner), b[0],
+              b[1], b[2], b[3]);
+  }
+
+  // ---- stage 1: T[k][16 rank + x], to the first CTA; stage 2 there, by the same code:
+  // P[x][y] = sum over m of T[x][m] D[y][m]
+  if (warp < 4) {
+    ok &= mbar_wait(&sm.dt_full, 0, abort_flag);
+#pragma unroll 1
+    for (int stage = 0; stage < (rank == 0 ? 2 : 1); ++stage) {
+      ok &= mbar_wait(&sm.in_full[stage], 0, abort_flag);
+      split_dct_stage(sm, stage, rank, warp, lane, prm.neg_zero);
+      __syncwarp();
+    }
+  }
+  cluster_arrive_relaxed();  // waited for at the end: no CTA leaves while another may write to it
+  if (!ok && lane == 0) {
+    // data did not land in time: the outputs are not trustworthy. Give this warp's copy a
+    // last bounded wait before the CTA may exit.
+    *abort_flag = 1;
+    atomicOr(prm.dev_err, kDevErrTimeout);
+    const uint64_t t0 = globaltimer_ns();
+    while (!mbar_try_wait(&sm.full[g], 0) && globaltimer_ns() - t0 < kWaitLimitNs / 4) {
+    }
+  }
+  if (rank == 0) {
+    __syncthreads();
+    if (warp < 8) {
+      if (prm.quality)
+        split_quality(sm.p[0], warp, prm.row_mask, prm.col_mask, lane, sm.grad[warp],
+                      prm.quality + n * 8);
+    } else if (warp < 12) {
+      EpilogueOut o;
+      o.hashes = prm.hashes ? prm.hashes + n * 256 : nullptr;
+      o.quality = nullptr;
+      o.thresholds = prm.thresholds ? prm.thresholds + n * 8 : nullptr;
+      o.pdqf_slots = prm.pdqf_slots;
+      o.pdqf = prm.pdqf ? prm.pdqf + n * (prm.pdqf_slots == 8 ? 8 : 1) * 256 : nullptr;
+      split_slots(sm.p[0], warp - 8, prm.row_mask, prm.col_mask, lane, o);
+    }
+  }
+  cluster_wait();
+}
+
 // Dihedrals of given PDQF matrices: one warp per matrix.
 __global__ void __launch_bounds__(128) dihedral_kernel(const DihedralLaunch prm) {
   __shared__ __align__(16) float P[4][256];
@@ -1110,27 +1538,74 @@ struct LaunchOne {
   }
 };
 
+template <typename Tin>
+static size_t split_smem_bytes() {
+  return kSplitRowsOffset + kSplitInRows * InputTraits<Tin>::kRowBytes + 128;  // + base alignment
+}
+template <typename Tin>
+static cudaError_t set_split_smem() {
+  return cudaFuncSetAttribute(hash_split_kernel<Tin>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(split_smem_bytes<Tin>()));
+}
+template <typename Tin>
+static cudaError_t launch_split(HashLaunch p, cudaStream_t s) {
+  p.neg_zero = -0.0f;
+  hash_split_kernel<Tin><<<static_cast<unsigned>(kSplitCtas * p.n), kSplitThreads,
+                           split_smem_bytes<Tin>(), s>>>(p);
+  return cudaGetLastError();
+}
+
+// Largest batch that hash_split_kernel takes. Its time grows with the waves of clusters (16 or
+// more images at once), hash_kernel's steps with the CTAs per SM: 41 us (f32, u8; RGB 80 us)
+// up to 152 images, 47-51 us (95-97 us) up to 304. Measured on both sides, split against
+// persistent: f32 39.4 / 41.3 us at 88 and 43.7 / 41.3 at 96 images; u8 46.9 / 50.7 at 208
+// and 49.6 / 50.5 at 224; RGB8 91.2 / 96.7 at 192 and 97.7 / 96.6 at 208; RGBA8 88.2 / 96.7
+// at 176 and 95.2 / 97.2 at 192.
+static int64_t split_max_images(int input_kind) {
+  switch (input_kind) {
+    case YPDQ_INPUT_F32: return 88;
+    case YPDQ_INPUT_U8: return 208;
+    case YPDQ_INPUT_RGB8: return 184;
+    default: return 176;
+  }
+}
+
 cudaError_t hash_occupancy_variant(int input_kind, int dct, int separable, int* ctas_per_sm) {
   return dispatch<OccupancyOf>(input_kind, dct, separable, ctas_per_sm);
 }
 
 cudaError_t launch_hash(const HashLaunch& p, int num_sms, int ctas_per_sm, cudaStream_t s) {
   if (p.n <= 0) return cudaSuccess;
+  if (p.dct == 0 && !p.separable && p.n <= split_max_images(p.input_kind)) {
+    switch (p.input_kind) {
+      case YPDQ_INPUT_F32: return launch_split<float>(p, s);
+      case YPDQ_INPUT_U8: return launch_split<uint8_t>(p, s);
+      case YPDQ_INPUT_RGB8: return launch_split<rgb8_t>(p, s);
+      case YPDQ_INPUT_RGBA8: return launch_split<rgba8_t>(p, s);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   int64_t grid = static_cast<int64_t>(num_sms) * (ctas_per_sm > 0 ? ctas_per_sm : 1);
   if (grid > p.n) grid = p.n;
   return dispatch<LaunchOne>(p.input_kind, p.dct, p.separable, p, grid, s);
 }
 
 cudaError_t upload_constants() {
-  float d[16 * 127];
+  float d[16 * 127], dt[128 * 16] = {};
   for (int i = 0; i < 16 * 127; ++i) {
     uint32_t b = YPDQ_DCT_F32_BITS[i];
     memcpy(&d[i], &b, 4);
+    dt[(i % 127) * 16 + i / 127] = d[i];
   }
   cudaError_t e = cudaMemcpyToSymbol(g_dct, d, sizeof(d));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_dct_t, dt, sizeof(dt));
   for (int kind = 0; kind < 4 && e == cudaSuccess; ++kind)
     for (int dct = 0; dct < 3 && e == cudaSuccess; ++dct)
       for (int sep = 0; sep < 2 && e == cudaSuccess; ++sep) e = dispatch<SetSmemAttr>(kind, dct, sep);
+  if (e == cudaSuccess) e = set_split_smem<float>();
+  if (e == cudaSuccess) e = set_split_smem<uint8_t>();
+  if (e == cudaSuccess) e = set_split_smem<rgb8_t>();
+  if (e == cudaSuccess) e = set_split_smem<rgba8_t>();
   return e;
 }
 

@@ -188,6 +188,7 @@ struct HashLaunch {
   int separable;  // nonzero: separable compress (YPDQ_COMPRESS_SEPARABLE) instead of the
                   // reference's tap order
   const int64_t* n_dev;  // if set, the image count is read from here (graph replay); n is the bound
+  float neg_zero;        // -0.0f, set by launch_hash: a constant the compiler does not know
 };
 
 struct DihedralLaunch {
