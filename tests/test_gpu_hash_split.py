@@ -8,8 +8,9 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-CASES = [("f32", n) for n in (1, 2, 88, 89)] + [("u8", n) for n in (1, 208, 209)] + \
-        [("rgb8", n) for n in (1, 184, 185)] + [("rgba8", n) for n in (1, 176, 177)]
+CASES = [("f32", n) for n in (1, 2, 56, 57, 88, 89)] + \
+        [("u8", n) for n in (1, 104, 105, 208, 209)] + \
+        [("rgb8", n) for n in (1, 72, 73, 184, 185)] + [("rgba8", n) for n in (1, 72, 73, 176, 177)]
 
 
 def images_of(yp, kind, n):

@@ -22,9 +22,21 @@
 //              accumulates DCT stage 1 (16 x 127 x 127) as each compressed row appears,
 //              then computes the 16 x 16 stage 2 together.
 //   warp 4     producer: one lane streams the image into a shared-memory ring with 1-D
-//              bulk async copies (4 input rows = one stage), NSTAGE stages deep.
+//              bulk async copies (8 or 16 input rows = one stage), a few stages deep.
 //   warp 5     epilogue: quality, exact medians, bits and dihedrals of image k while the
 //              compute warps already work on image k+1 (double-buffered PDQF).
+//
+// f32 input is bound by HBM (1,024 images 168 us, 6.4 TB/s). The others are bound by issue
+// slots (64 % busy with the two compute warps per scheduler that 167 registers allow), so
+// what counts is instructions per compressed value, ~130 of which 27 are its serial sum:
+//   * a 4-row group finishes one value and starts the next from one carried sum, so nothing
+//     is read or converted twice and a stage of 2-4 groups costs one wait and one release;
+//   * byte conversion and product are one fma, products and DCT accumulators go in packed
+//     pairs (an f32x2 instruction takes two cycles of the FMA pipe but one issue slot);
+//   * RGB pixels become luma where they are read, without a staging of their own.
+// 4,096 u8 images: 552 -> 375 us (10.9 M images/s); 801 RGB8 images 262 -> 154 us; u8 with
+// the separable compress and the BF16x3 DCT, 1,024 images: 133 -> 83 us. A third CTA per SM
+// (96 registers, spilling) was slower: 434 us.
 #include <cuda_bf16.h>
 
 #include <cstring>
@@ -39,14 +51,14 @@ namespace ypdq {
 __device__ float g_dct[16 * 127];  // D[k][i] = sqrt(2/127) cos(pi (k+1) (2i+1) / 254), f32
 __device__ alignas(16) float g_dct_t[128 * 16];  // the same as D^T: [i][k]; row 127 is zero
 
-constexpr int kStagesPerImage = 128;  // stage s holds rows 4s+1 .. 4s+4 (stage 127: 509, 510)
+constexpr int kGroupsPerImage = 128;  // group g holds rows 4g+1 .. 4g+4 (group 127: 509, 510)
 constexpr int kComputeThreads = 128;
 constexpr int kProducerWarp = 4;
 constexpr int kEpilogueWarp = 5;
 constexpr int kMmaWarpHash = 6;   // tensor-core DCT only: allocates TMEM, issues the MMAs
 template <int kDct>
 constexpr int hash_threads() { return kDct == 0 ? 192 : 224; }
-// RGB8 / RGBA8 pixels, converted to f32 luma once per stage (see convert_stage).
+// RGB8 / RGBA8 pixels, converted to f32 luma where they are read (see load_row).
 struct rgb8_t {
   uint8_t c[3];
 };
@@ -58,31 +70,17 @@ constexpr bool is_rgb() {
   return std::is_same<Tin, rgb8_t>::value || std::is_same<Tin, rgba8_t>::value;
 }
 
-// Depth of the input ring (4-row stages). The tensor-core variants with f32 input use 6
-// stages so that two CTAs fit on an SM next to their operand buffers.
-#ifndef YPDQ_RING_U8
-#define YPDQ_RING_U8 8
-#endif
-#ifndef YPDQ_RING_U8_TC
-#define YPDQ_RING_U8_TC 16
-#endif
-#ifndef YPDQ_U8_TC_CTAS
-#define YPDQ_U8_TC_CTAS 2
-#endif
+// A stage of the input ring is one bulk copy of kGroups groups of 4 rows: the compute warps
+// wait once for it and free it once, so a wider stage spreads that over more rows, as far as
+// a few stages in flight still fit beside each other. In bytes per CTA: u8 4 x 8 KB, RGB8
+// 6 (tensor-core DCT: 3) x 12 KB, f32 and RGBA8 5 (3) x 16 KB.
+template <typename Tin>
+constexpr int stage_groups() { return sizeof(Tin) == 1 ? 4 : 2; }
 template <typename Tin, int kDct>
 constexpr int ring_stages() {
-  return is_rgb<Tin>() ? (kDct != 0 ? 3 : 6)
-                       : (sizeof(Tin) == 4 ? (kDct != 0 ? 6 : 8)
-                                           : (kDct != 0 ? YPDQ_RING_U8_TC : YPDQ_RING_U8));
+  return sizeof(Tin) == 1 ? 4 : kDct != 0 ? 3 : sizeof(Tin) == 3 ? 6 : 5;
 }
-template <typename Tin>
-constexpr int conv_slots() { return is_rgb<Tin>() ? 3 : 0; }
-// The tensor-core variants need no DCT accumulators in registers: with u8 input (issue-
-// bound, not HBM-bound) they run 3 CTAs per SM.
-template <typename Tin, int kDct>
-constexpr int hash_min_blocks() { return (kDct != 0 && sizeof(Tin) == 1) ? YPDQ_U8_TC_CTAS : 2; }
 constexpr int kComputeBarrier = 1;  // named barrier id used by the 128 compute threads
-constexpr int kConvRow = 136;       // floats per row of an RGB luma staging (128 + 4, padded)
 
 // Stage 1 of the DCT on tensor cores (kDct = 1: TF32, 2: BF16x3). The compressed values
 // are written, chunk by chunk of compressed rows, into a 128-byte-swizzled K-major operand
@@ -111,16 +109,12 @@ struct DctTraits<2> {  // BF16x3: 32 rows x 2 B (64-byte swizzle), hi at +0 and 
   static constexpr int kALo = 8192, kDLo = 4096;  // byte offsets of the lo operands
 };
 
-template <int kStageBytes, int kNumStages, int kDct, int kConvSlots>
+template <int kStageBytes, int kNumStages, int kDct>
 struct HashSmem {
-  // RGB input only: per compute warp, f32 luma of its columns of the last 3 stages
-  alignas(16) float conv[kConvSlots > 0 ? 4 : 1][kConvSlots > 0 ? kConvSlots : 1]
-                        [kConvSlots > 0 ? 4 * kConvRow : 4];
   alignas(1024) uint8_t ops[2][DctTraits<kDct>::kBufBytes];  // A operand, double-buffered
   alignas(1024) uint8_t dops[DctTraits<kDct>::kDBytes];      // B operand (DCT matrix)
   alignas(128) unsigned char ring[kNumStages][kStageBytes];
-  alignas(16) float dt[kDct == 0 ? 128 : 1][16];  // dt[i][k] = D[k][i]; row 127 is zero
-  float dr[16][129];              // D[k][m], padded against bank conflicts
+  alignas(16) float dt[128][16];  // dt[i + 1][k] = D[k][i]; row 0 is zero
   float t[16][129];               // DCT stage 1 result T = D * B
   alignas(16) float p[2][256];    // PDQF, double-buffered between compute and epilogue
   uint64_t full[kNumStages];
@@ -150,16 +144,6 @@ template <>
 struct InputTraits<rgba8_t> {
   static constexpr int kRowBytes = 512 * 4;
 };
-// The element type the compress reads: the input itself, or f32 luma for RGB input.
-template <typename Tin, bool kRgb = is_rgb<Tin>()>
-struct CompressIn {
-  using T = Tin;
-};
-template <typename Tin>
-struct CompressIn<Tin, true> {
-  using T = float;
-};
-
 // Two f32 operations in one instruction, each rounded by itself. ptxas (13.0) contracts a
 // packed multiply and the packed add that takes its result into one fused operation, .rn or
 // not (scalar mul.rn / add.rn it leaves alone), which would change bits. So a product is
@@ -177,6 +161,15 @@ __device__ __forceinline__ float2 fma2_rn(float2 a, float2 b, float2 c) {
 __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b, float neg_zero) {
   return fma2_rn(a, b, make_float2(neg_zero, neg_zero));
 }
+// The plain packed multiply, for products that only scalar adds take.
+__device__ __forceinline__ float2 mul2_contractible_rn(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 __device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
   float2 d;
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
@@ -186,150 +179,136 @@ __device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
   return d;
 }
 
+// Byte k (0..3) of w as the float 2^23 + byte, placed in the mantissa by a byte permute. A
+// product with a weight takes the 2^23 off again in its own rounding: RN(W byte) is
+// fma(W, 2^23 + byte, -2^23 W), one instruction for the conversion and the product, exact
+// before the rounding because 2^23 W is (no I2F on the quarter-rate pipe either).
+constexpr float kByteBias = 8388608.0f;
+template <int k>
+__device__ __forceinline__ float byte_biased(uint32_t w) {
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 | k));
+}
+template <int k>
+__device__ __forceinline__ float byte_f(uint32_t w) {
+  return byte_biased<k>(w) - kByteBias;
+}
 // ITU-R BT.601 luma in the reference's scalar order (Kernel::cvt_rgb8_to_luma8f,
 // src/kernel/mod.rs:303-340, coefficients src/kernel/constants.rs:23):
 // (0.299 r + 0.587 g) + 0.114 b, each product and sum rounded to f32, no fused multiply-add.
-__device__ __forceinline__ float luma_bt601(float r, float g, float b) {
-  return __fadd_rn(__fadd_rn(__fmul_rn(0.299f, r), __fmul_rn(0.587f, g)), __fmul_rn(0.114f, b));
+// Two pixels at once, from biased bytes.
+__device__ __forceinline__ float2 luma2_bt601(float2 r, float2 g, float2 b) {
+  constexpr float cr = 0.299f, cg = 0.587f, cb = 0.114f;
+  const float2 pr = fma2_rn(r, make_float2(cr, cr), make_float2(-kByteBias * cr, -kByteBias * cr));
+  const float2 pg = fma2_rn(g, make_float2(cg, cg), make_float2(-kByteBias * cg, -kByteBias * cg));
+  const float2 pb = fma2_rn(b, make_float2(cb, cb), make_float2(-kByteBias * cb, -kByteBias * cb));
+  return add2_rn(add2_rn(pr, pg), pb);
 }
-// Byte k (0..3) of w as an exact float: the byte placed in the mantissa of 2^23 by a byte
-// permute, then 2^23 subtracted (keeps the conversion off the quarter-rate I2F path).
-template <int k>
-__device__ __forceinline__ float byte_f(uint32_t w) {
-  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 | k)) - 8388608.0f;
+// Pixels 0-1 and 2-3 of four: RGB8 in three words (r g b r | g b r g | b r g b), RGBA8 in four.
+__device__ __forceinline__ float2 luma01(uint32_t a, uint32_t b, uint32_t) {
+  return luma2_bt601(make_float2(byte_biased<0>(a), byte_biased<3>(a)),
+                     make_float2(byte_biased<1>(a), byte_biased<0>(b)),
+                     make_float2(byte_biased<2>(a), byte_biased<1>(b)));
 }
-// Luma staging of one 4-row stage for one compute warp: warp w reads input columns
-// 128w .. 128w+131 (its 32 compressed columns need 4j .. 4j+7), stored as 4 rows of
-// kConvRow floats from column 128w on. Lane l converts columns 128w+4l .. +3 of each row;
-// lanes 0..15 also convert the 4 columns past the warp's 128 (row l/4), 0 past the image.
-__device__ __forceinline__ uint32_t rgb_word(const unsigned char* p) {  // 4-byte aligned
-  return *reinterpret_cast<const uint32_t*>(p);
+__device__ __forceinline__ float2 luma23(uint32_t, uint32_t b, uint32_t c) {
+  return luma2_bt601(make_float2(byte_biased<2>(b), byte_biased<1>(c)),
+                     make_float2(byte_biased<3>(b), byte_biased<2>(c)),
+                     make_float2(byte_biased<0>(c), byte_biased<3>(c)));
 }
-template <typename Tin>
-__device__ __forceinline__ void convert_stage_warp(const unsigned char* raw, float* out, int w,
-                                                   int lane) {
-  constexpr int kRowBytes = InputTraits<Tin>::kRowBytes;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int c0 = 128 * w + 4 * lane;
-    const unsigned char* row = raw + r * kRowBytes;
-    float l[4];
-    if constexpr (sizeof(Tin) == 4) {
-      const uint4 v = *reinterpret_cast<const uint4*>(row + 4 * c0);
-      const uint32_t px[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) l[k] = luma_bt601(byte_f<0>(px[k]), byte_f<1>(px[k]), byte_f<2>(px[k]));
-    } else {
-      const unsigned char* p = row + 3 * c0;  // 12 bytes: r g b r | g b r g | b r g b
-      const uint32_t a = rgb_word(p), b = rgb_word(p + 4), c = rgb_word(p + 8);
-      l[0] = luma_bt601(byte_f<0>(a), byte_f<1>(a), byte_f<2>(a));
-      l[1] = luma_bt601(byte_f<3>(a), byte_f<0>(b), byte_f<1>(b));
-      l[2] = luma_bt601(byte_f<2>(b), byte_f<3>(b), byte_f<0>(c));
-      l[3] = luma_bt601(byte_f<1>(c), byte_f<2>(c), byte_f<3>(c));
-    }
-    *reinterpret_cast<float4*>(out + r * kConvRow + 4 * lane) = make_float4(l[0], l[1], l[2], l[3]);
-  }
-  if (lane < 16) {
-    const int r = lane >> 2, c = 128 * w + 128 + (lane & 3);
-    float v = 0.0f;
-    if (c < 512) {
-      const unsigned char* p = raw + r * kRowBytes + c * static_cast<int>(sizeof(Tin));
-      v = luma_bt601(static_cast<float>(p[0]), static_cast<float>(p[1]), static_cast<float>(p[2]));
-    }
-    out[r * kConvRow + 128 + (lane & 3)] = v;
-  }
+__device__ __forceinline__ float2 luma_rgba(uint32_t p, uint32_t q) {
+  return luma2_bt601(make_float2(byte_biased<0>(p), byte_biased<0>(q)),
+                     make_float2(byte_biased<1>(p), byte_biased<1>(q)),
+                     make_float2(byte_biased<2>(p), byte_biased<2>(q)));
 }
-
-// Columns 4j .. 4j+7 of one input row held in shared memory.
-__device__ __forceinline__ void load_row8(const float* row, int j, float x[8]) {
+// The five columns 4j + 2 .. 4j + 6 of one input row in shared memory that compressed column
+// j reads: two pairs and one. f32 input and luma as they are, u8 biased (byte_biased).
+struct RowX {
+  float2 a, b;
+  float c;
+};
+__device__ __forceinline__ RowX load_row(const float* row, int j) {
   const float4* r = reinterpret_cast<const float4*>(row);
-  float4 a = r[j], b = r[j + 1];
-  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-  x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  const float4 a = r[j], b = r[j + 1];
+  return {make_float2(a.z, a.w), make_float2(b.x, b.y), b.z};
 }
-// u8 columns as exact floats through a byte permute and one add (byte_f), which keeps the
-// 27 conversions per compressed value off the quarter-rate conversion pipe.
-__device__ __forceinline__ void load_row8(const uint8_t* row, int j, float x[8]) {
+__device__ __forceinline__ RowX load_row(const uint8_t* row, int j) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(row);
-  uint32_t a = r[j], b = r[j + 1];
-  x[0] = byte_f<0>(a); x[1] = byte_f<1>(a); x[2] = byte_f<2>(a); x[3] = byte_f<3>(a);
-  x[4] = byte_f<0>(b); x[5] = byte_f<1>(b); x[6] = byte_f<2>(b); x[7] = byte_f<3>(b);
+  const uint32_t a = r[j], b = r[j + 1];
+  return {make_float2(byte_biased<2>(a), byte_biased<3>(a)),
+          make_float2(byte_biased<0>(b), byte_biased<1>(b)), byte_biased<2>(b)};
 }
-
-// RGB columns as f32 luma, converted on load (hash_split_kernel; hash_kernel converts whole
-// stages once instead, see convert_stage_warp).
-__device__ __forceinline__ void load_row8(const rgb8_t* row, int j, float x[8]) {
+// RGB columns as f32 luma, converted on load (9 of 8 columns' work: each column is read by
+// 1.25 threads). Converting whole stages into a luma staging first cost more: its stores,
+// its loads and a barrier per row.
+__device__ __forceinline__ RowX load_row(const rgb8_t* row, int j) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(row) + 3 * j;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {  // 12 bytes each: r g b r | g b r g | b r g b
-    const uint32_t a = r[3 * h], b = r[3 * h + 1], c = r[3 * h + 2];
-    x[4 * h + 0] = luma_bt601(byte_f<0>(a), byte_f<1>(a), byte_f<2>(a));
-    x[4 * h + 1] = luma_bt601(byte_f<3>(a), byte_f<0>(b), byte_f<1>(b));
-    x[4 * h + 2] = luma_bt601(byte_f<2>(b), byte_f<3>(b), byte_f<0>(c));
-    x[4 * h + 3] = luma_bt601(byte_f<1>(c), byte_f<2>(c), byte_f<3>(c));
-  }
+  return {luma23(r[0], r[1], r[2]), luma01(r[3], r[4], r[5]), luma23(r[3], r[4], r[5]).x};
 }
-__device__ __forceinline__ void load_row8(const rgba8_t* row, int j, float x[8]) {
+__device__ __forceinline__ RowX load_row(const rgba8_t* row, int j) {
   const uint4* r = reinterpret_cast<const uint4*>(row);
   const uint4 a = r[j], b = r[j + 1];
-  const uint32_t px[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    x[k] = luma_bt601(byte_f<0>(px[k]), byte_f<1>(px[k]), byte_f<2>(px[k]));
+  return {luma_rgba(a.z, a.w), luma_rgba(b.x, b.y), luma_rgba(b.z, b.z).x};
 }
 
 #define YPDQ_W(di, dj) __uint_as_float(YPDQ_TENT_BITS_##di##_##dj)
-#define YPDQ_TAP(acc, di, dj, x) acc = __fadd_rn(acc, __fmul_rn(YPDQ_W(di, dj), (x)))
-#define YPDQ_ROW_TAPS(acc, di, x)     \
-  YPDQ_TAP(acc, di, 1, x[2]);         \
-  YPDQ_TAP(acc, di, 2, x[3]);         \
-  YPDQ_TAP(acc, di, 3, x[4]);         \
-  YPDQ_TAP(acc, di, 4, x[5]);         \
-  YPDQ_TAP(acc, di, 5, x[6])
+// The weights of a tap row are (w1, w2, w3, w2, w1), and rows 1, 2 equal rows 5, 4.
+static_assert(YPDQ_TENT_BITS_1_1 == YPDQ_TENT_BITS_1_5 && YPDQ_TENT_BITS_1_2 == YPDQ_TENT_BITS_1_4 &&
+              YPDQ_TENT_BITS_2_1 == YPDQ_TENT_BITS_2_5 && YPDQ_TENT_BITS_2_2 == YPDQ_TENT_BITS_2_4 &&
+              YPDQ_TENT_BITS_3_1 == YPDQ_TENT_BITS_3_5 && YPDQ_TENT_BITS_3_2 == YPDQ_TENT_BITS_3_4 &&
+              YPDQ_TENT_BITS_1_1 == YPDQ_TENT_BITS_5_1 && YPDQ_TENT_BITS_1_2 == YPDQ_TENT_BITS_5_2 &&
+              YPDQ_TENT_BITS_1_3 == YPDQ_TENT_BITS_5_3 && YPDQ_TENT_BITS_5_1 == YPDQ_TENT_BITS_5_5 &&
+              YPDQ_TENT_BITS_5_2 == YPDQ_TENT_BITS_5_4 && YPDQ_TENT_BITS_2_1 == YPDQ_TENT_BITS_4_1 &&
+              YPDQ_TENT_BITS_2_2 == YPDQ_TENT_BITS_4_2 && YPDQ_TENT_BITS_2_3 == YPDQ_TENT_BITS_4_3 &&
+              YPDQ_TENT_BITS_4_1 == YPDQ_TENT_BITS_4_5 && YPDQ_TENT_BITS_4_2 == YPDQ_TENT_BITS_4_4,
+              "the tent table is symmetric");
 
-// Compressed value (i, j) in the reference's tap order: rows 4i+1 .. 4i+6 come from stage i
-// (rows 0..3) and stage i+1 (rows 0..1); tap (di, dj) reads input column 4j+1+dj, which is
-// x[1+dj]; row 4i+1 holds only the two residue taps. Called for consecutive output rows of
-// one column: the first two input rows of output row i + 1 (4i + 5, 4i + 6) are the last
-// two of row i, so their converted values (x[5], x[6] of the first; x[2..6] of the second)
-// stay in registers instead of being read and converted twice.
-struct CompressCarry {
-  float a5, a6;   // row 4i + 1: the residue taps' inputs
-  float b[5];     // row 4i + 2: x[2..6]
+// RN(w x) of one value and of a whole tap row. The sums that take the products are scalar
+// adds (a packed multiply is only contracted with a packed add).
+template <typename T>
+__device__ __forceinline__ float weighted(float w, float x) {
+  if constexpr (sizeof(T) == 1) return __fmaf_rn(w, x, -kByteBias * w);
+  else return __fmul_rn(w, x);
+}
+template <typename T>
+__device__ __forceinline__ float2 weighted2(float w0, float w1, float2 x) {
+  const float2 w = make_float2(w0, w1);
+  if constexpr (sizeof(T) == 1) return fma2_rn(w, x, make_float2(-kByteBias * w0, -kByteBias * w1));
+  else return mul2_contractible_rn(w, x);
+}
+template <typename T>
+__device__ __forceinline__ RowX weighted_row(float w1, float w2, float w3, const RowX& x) {
+  return {weighted2<T>(w1, w2, x.a), weighted2<T>(w3, w2, x.b), weighted<T>(w1, x.c)};
+}
+__device__ __forceinline__ float add_row(float s, const RowX& p) {
+  return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, p.a.x), p.a.y), p.b.x), p.b.y), p.c);
+}
+
+// The compress walks a column group by group. Compressed value i takes rows 4i + 1 .. 4i + 6
+// in the reference's tap order; row 4i + 1 holds only the two residue taps (columns 4j + 5
+// and 4j + 6). Group g's rows 4g + 1 and 4g + 2 are the last two of value g - 1 and the first
+// two of value g, and its rows 4g + 3 and 4g + 4 the next two of value g. So one group
+// finishes value g - 1 from the sum carried over and starts value g, with nothing but that
+// sum between groups; the products of row 4g + 2 serve both values (tap rows 1 and 5 have
+// equal weights).
+struct TapSum {
+  float s = 0.0f;  // value g through tap row 3
 };
-template <typename Tin, int kRow = 512>
-__device__ __forceinline__ float compress_next(const Tin* st0, const Tin* st1, int j, bool first,
-                                               CompressCarry& c) {
-  float x[8];
-  float s = 0.0f;
-  if (first) {
-    load_row8(st0 + 0 * kRow, j, x);
-    c.a5 = x[5];
-    c.a6 = x[6];
-    load_row8(st0 + 1 * kRow, j, x);
-#pragma unroll
-    for (int e = 0; e < 5; ++e) c.b[e] = x[2 + e];
+template <typename Tin>
+__device__ __forceinline__ float compress_group(const Tin* rows, int j, bool last, TapSum& c) {
+  using T = typename std::conditional<is_rgb<Tin>(), float, Tin>::type;
+  const RowX x = load_row(rows, j);
+  const RowX p = weighted_row<T>(YPDQ_W(1, 1), YPDQ_W(1, 2), YPDQ_W(1, 3), load_row(rows + 512, j));
+  const RowX p4 = weighted_row<T>(YPDQ_W(4, 1), YPDQ_W(4, 2), YPDQ_W(4, 3), x);
+  const float done = add_row(add_row(c.s, p4), p);
+  if (!last) {
+    float s = __fadd_rn(__fadd_rn(0.0f, weighted<T>(YPDQ_W(0, 4), x.b.y)),
+                        weighted<T>(YPDQ_W(0, 5), x.c));
+    s = add_row(s, p);
+    s = add_row(s, weighted_row<T>(YPDQ_W(2, 1), YPDQ_W(2, 2), YPDQ_W(2, 3),
+                                   load_row(rows + 2 * 512, j)));
+    c.s = add_row(s, weighted_row<T>(YPDQ_W(3, 1), YPDQ_W(3, 2), YPDQ_W(3, 3),
+                                     load_row(rows + 3 * 512, j)));
   }
-  YPDQ_TAP(s, 0, 4, c.a5);
-  YPDQ_TAP(s, 0, 5, c.a6);
-  YPDQ_TAP(s, 1, 1, c.b[0]);
-  YPDQ_TAP(s, 1, 2, c.b[1]);
-  YPDQ_TAP(s, 1, 3, c.b[2]);
-  YPDQ_TAP(s, 1, 4, c.b[3]);
-  YPDQ_TAP(s, 1, 5, c.b[4]);
-  load_row8(st0 + 2 * kRow, j, x);
-  YPDQ_ROW_TAPS(s, 2, x);
-  load_row8(st0 + 3 * kRow, j, x);
-  YPDQ_ROW_TAPS(s, 3, x);
-  load_row8(st1 + 0 * kRow, j, x);
-  YPDQ_ROW_TAPS(s, 4, x);
-  c.a5 = x[5];
-  c.a6 = x[6];
-  load_row8(st1 + 1 * kRow, j, x);
-  YPDQ_ROW_TAPS(s, 5, x);
-#pragma unroll
-  for (int e = 0; e < 5; ++e) c.b[e] = x[2 + e];
-  return s;
+  return done;
 }
 
 // Separable compress (YPDQ_COMPRESS_SEPARABLE; not the reference's operation order). The
@@ -338,35 +317,30 @@ __device__ __forceinline__ float compress_next(const Tin* st0, const Tin* st1, i
 //   out[i][j] = S / 81,  S = sum_{r = 2..6} c[r] h(4i + r),  h(row) = sum_{k = 2..6} c[k] x[row][4j + k]
 // Each h row serves two output rows. For u8 input h and S are exact integers (two dp4a per
 // h), so the only rounding is the final scale.
-__device__ __forceinline__ float hsum(const uint8_t* row, int j) {
-  const uint32_t* r = reinterpret_cast<const uint32_t*>(row);
-  // bytes of r[j]: columns 4j .. 4j+3 (weights 0, 0, 1, 2); r[j+1]: 4j+4 .. 4j+7 (3, 2, 1, 0)
-  return static_cast<float>(__dp4a(r[j], 0x02010000u, __dp4a(r[j + 1], 0x00010203u, 0u)));
+template <typename Tin>
+__device__ __forceinline__ float hsum(const Tin* row, int j) {
+  if constexpr (std::is_same<Tin, uint8_t>::value) {
+    const uint32_t* r = reinterpret_cast<const uint32_t*>(row);
+    // bytes of r[j]: columns 4j .. 4j+3 (weights 0, 0, 1, 2); r[j+1]: 4j+4 .. 4j+7 (3, 2, 1, 0)
+    return static_cast<float>(__dp4a(r[j], 0x02010000u, __dp4a(r[j + 1], 0x00010203u, 0u)));
+  } else {
+    const RowX x = load_row(row, j);
+    return (x.a.x + x.c) + 2.0f * (x.a.y + x.b.y) + 3.0f * x.b.x;
+  }
 }
-__device__ __forceinline__ float hsum(const float* row, int j) {
-  const float4* r = reinterpret_cast<const float4*>(row);
-  const float4 a = r[j], b = r[j + 1];  // columns 4j .. 4j+3 and 4j+4 .. 4j+7
-  return (a.z + b.z) + 2.0f * (a.w + b.y) + 3.0f * b.x;
-}
-// h of rows 1..3 of a 4-row stage (rows 4s+2 .. 4s+4), carried to the next output row.
+// h of rows 4g + 2 .. 4g + 4, carried to the group that finishes value g.
 struct HCarry {
-  float h1, h2, h3;
+  float h1 = 0.0f, h2 = 0.0f, h3 = 0.0f;
 };
-template <typename Tin, int kRow = 512>
-__device__ __forceinline__ void hcarry_init(const Tin* st, int j, HCarry& c) {
-  c.h1 = hsum(st + 1 * kRow, j);
-  c.h2 = hsum(st + 2 * kRow, j);
-  c.h3 = hsum(st + 3 * kRow, j);
-}
-// Output row i from the carried h of stage i and the new stage i+1 (rows 4i+5 .. 4i+8).
-template <typename Tin, int kRow = 512>
-__device__ __forceinline__ float compress_separable(const Tin* st1, int j, HCarry& c) {
-  const float n0 = hsum(st1 + 0 * kRow, j), n1 = hsum(st1 + 1 * kRow, j);
-  const float n2 = hsum(st1 + 2 * kRow, j), n3 = hsum(st1 + 3 * kRow, j);
+template <typename Tin>
+__device__ __forceinline__ float compress_group(const Tin* rows, int j, bool last, HCarry& c) {
+  const float n0 = hsum(rows, j), n1 = hsum(rows + 512, j);
   const float S = (c.h1 + n1) + 2.0f * (c.h2 + n0) + 3.0f * c.h3;
-  c.h1 = n1;
-  c.h2 = n2;
-  c.h3 = n3;
+  if (!last) {
+    c.h1 = n1;
+    c.h2 = hsum(rows + 2 * 512, j);
+    c.h3 = hsum(rows + 3 * 512, j);
+  }
   return S * (1.0f / 81.0f);
 }
 
@@ -616,25 +590,16 @@ __device__ __forceinline__ void tmem_take16(uint32_t (&r)[16]) {
                  "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]));
 }
 
-// The compress input of global stage g: the ring slot itself, or (RGB) its luma slot.
-// (for RGB: the calling warp's staging, which starts at input column 128 * warp, so the
-// compress reads it at column index j - 32 * warp with rows kConvRow apart)
-template <typename Tin, typename CT, int kNumStages, typename Smem>
-__device__ __forceinline__ const CT* stage_ptr(Smem& sm, uint32_t g, int warp) {
-  if constexpr (is_rgb<Tin>()) return sm.conv[warp][g % 3];
-  else return reinterpret_cast<const CT*>(sm.ring[g % kNumStages]);
-}
-
 template <typename Tin, int kDct, bool kSep>
-__global__ void __launch_bounds__(hash_threads<kDct>(), (hash_min_blocks<Tin, kDct>()))
+__global__ void __launch_bounds__(hash_threads<kDct>(), 2)
     hash_kernel(const HashLaunch prm) {
   constexpr int kRowBytes = InputTraits<Tin>::kRowBytes;
-  constexpr int kStageBytes = 4 * kRowBytes;
+  constexpr int kGroups = stage_groups<Tin>();
+  constexpr int kStageBytes = 4 * kGroups * kRowBytes;
   constexpr int kNumStages = ring_stages<Tin, kDct>();
+  constexpr int kStagesPerImage = kGroupsPerImage / kGroups;
   constexpr int kThreads = hash_threads<kDct>();
-  using Smem = HashSmem<kStageBytes, kNumStages, kDct, conv_slots<Tin>()>;
-  constexpr bool kRgb = is_rgb<Tin>();
-  using CT = typename CompressIn<Tin>::T;
+  using Smem = HashSmem<kStageBytes, kNumStages, kDct>;
   extern __shared__ unsigned char smem_raw[];
   // Align by offsetting the shared array itself so the compiler keeps the shared address
   // space (an integer round trip would turn every access into a generic one).
@@ -645,13 +610,10 @@ __global__ void __launch_bounds__(hash_threads<kDct>(), (hash_min_blocks<Tin, kD
 
   for (int idx = tid; idx < 16 * 127; idx += kThreads) {
     const int k = idx / 127, i = idx - k * 127;
-    const float d = g_dct[idx];
-    if constexpr (kDct == 0) sm.dt[i][k] = d;
-    sm.dr[k][i] = d;
+    sm.dt[i + 1][k] = g_dct[idx];
   }
-  if constexpr (kDct == 0) {
-    if (tid < 16) sm.dt[127][tid] = 0.0f;
-  } else {
+  if (tid < 16) sm.dt[0][tid] = 0.0f;
+  if constexpr (kDct != 0) {
     // the DCT matrix as the MMA's B operand: N = 16 rows k, K = 128 (column 127 is zero)
     for (int idx = tid; idx < 16 * 128; idx += kThreads) {
       const int k = idx >> 7, i = idx & 127;
@@ -714,9 +676,10 @@ __global__ void __launch_bounds__(hash_threads<kDct>(), (hash_min_blocks<Tin, kD
           ok = false;
           break;
         }
-        const uint32_t bytes = (s < kStagesPerImage - 1) ? 4 * kRowBytes : 2 * kRowBytes;
+        // rows past 510 are read by no output
+        const uint32_t bytes = kStageBytes - (s < kStagesPerImage - 1 ? 0 : 2 * kRowBytes);
         mbar_arrive_expect_tx(&sm.full[slot], bytes);
-        bulk_g2s(sm.ring[slot], img + static_cast<int64_t>(4 * s + 1) * kRowBytes, bytes,
+        bulk_g2s(sm.ring[slot], img + kRowBytes + static_cast<int64_t>(s) * kStageBytes, bytes,
                  &sm.full[slot], policy);
       }
     }
@@ -832,188 +795,134 @@ __global__ void __launch_bounds__(hash_threads<kDct>(), (hash_min_blocks<Tin, kD
     }
   }
 
-  // ---- compute warps: thread j <-> compressed column j
-  const int j = tid;
+  // ---- compute warps: thread j <-> compressed column j (thread 127 repeats column 126 and
+  // drops it)
+  const int j = tid, jc = min(tid, 126);
   const bool active = j < 127;
-  // column index and row stride the compress reads with (RGB: the warp's own staging)
-  const int jc = kRgb ? lane : j;
-  constexpr int kCRow = kRgb ? kConvRow : 512;
-  uint32_t it = 0;
+  const float nz = prm.neg_zero;
+  uint32_t it = 0, slot = 0, phase = 0;  // the stage being read
   for (int64_t n = blockIdx.x; n < n_images; n += gridDim.x, ++it) {
-    const uint32_t g0 = it * kStagesPerImage;
-    if constexpr (kDct != 0) {
-      // stage 1 on tensor cores: write the compressed column into the operand chunks
-      constexpr int kR = DctTraits<kDct>::kRowsPerChunk;
-      constexpr uint32_t kChunks = 128 / kR;
-      const uint32_t gc0 = it * kChunks;
-      if (!mbar_wait(&sm.full[g0 % kNumStages], (g0 / kNumStages) & 1u, abort_flag)) goto fail;
-      if constexpr (kRgb) {
-        // the first stage to luma; the barrier also orders this image's slot writes after
-        // every thread's last read of the previous image
-        convert_stage_warp<Tin>(sm.ring[g0 % kNumStages], sm.conv[warp][g0 % 3], warp, lane);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.empty[g0 % kNumStages]);
-      }
-      HCarry hc{};
-      CompressCarry cc{};
-      if (kSep && active)
-        hcarry_init<CT, kCRow>(stage_ptr<Tin, CT, kNumStages>(sm, g0, warp), jc, hc);
-      for (int i0 = 0; i0 < 128; i0 += 4) {
-        float b[4];
+    typename std::conditional<kSep, HCarry, TapSum>::type carry;
+    float* const buf1 = prm.buf1 && active ? prm.buf1 + n * 127 * 128 + j : nullptr;
+    // FP32: the 16 x 4 accumulators [pair of frequencies][partial sum]
+    float2 acc[kDct == 0 ? 8 : 1][4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int i = i0 + r;
-          b[r] = 0.0f;
-          if (i < 127) {
-            const uint32_t ga = g0 + i, gb = ga + 1;
-            if (!mbar_wait(&sm.full[gb % kNumStages], (gb / kNumStages) & 1u, abort_flag))
-              goto fail;
-            if constexpr (kRgb) {
-              convert_stage_warp<Tin>(sm.ring[gb % kNumStages], sm.conv[warp][gb % 3], warp, lane);
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&sm.empty[gb % kNumStages]);
-            }
-            if (active) {
-              const CT* st0 = stage_ptr<Tin, CT, kNumStages>(sm, ga, warp);
-              const CT* st1 = stage_ptr<Tin, CT, kNumStages>(sm, gb, warp);
-              b[r] = kSep ? compress_separable<CT, kCRow>(st1, jc, hc)
-                          : compress_next<CT, kCRow>(st0, st1, jc, i == 0, cc);
-              if (prm.buf1) prm.buf1[(n * 127 + i) * 128 + j] = b[r];
-            }
-            if constexpr (!kRgb) {
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&sm.empty[ga % kNumStages]);
-            }
+    for (int k = 0; k < (kDct == 0 ? 8 : 1); ++k)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[k][r] = make_float2(0.0f, 0.0f);
+    // tensor cores: values 4 q - 4 .. 4 q - 1, written to the operand as one unit
+    float unit[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto write_unit = [&](int u) -> bool {  // rows 4 u .. 4 u + 3 of the operand
+      constexpr int kR = DctTraits<kDct>::kRowsPerChunk;
+      const uint32_t within = static_cast<uint32_t>(4 * u % kR);
+      const uint32_t chunk = it * (128 / kR) + static_cast<uint32_t>(4 * u / kR);
+      const uint32_t buf = chunk & 1;
+      if (within == 0 && !mbar_wait(&sm.a_empty[buf], ((chunk >> 1) & 1u) ^ 1u, abort_flag))
+        return false;
+      if constexpr (kDct == 1) {
+        const uint4 w = make_uint4(to_tf32(unit[0]), to_tf32(unit[1]), to_tf32(unit[2]), to_tf32(unit[3]));
+        *reinterpret_cast<uint4*>(sm.ops[buf] + sw128_offset(j, within, 4)) = w;
+      } else if constexpr (kDct == 2) {
+        uint32_t h01, l01, h23, l23;
+        split_bf16x2(unit[0], unit[1], h01, l01);
+        split_bf16x2(unit[2], unit[3], h23, l23);
+        const uint32_t off = sw64_offset(j, within, 2);
+        *reinterpret_cast<uint2*>(sm.ops[buf] + off) = make_uint2(h01, h23);
+        *reinterpret_cast<uint2*>(sm.ops[buf] + DctTraits<kDct>::kALo + off) = make_uint2(l01, l23);
+      }
+      if (within + 4 == static_cast<uint32_t>(kR)) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.a_full[buf]);
+      }
+      return true;
+    };
+    // groups 4 q .. 4 q + 3 finish values 4 q - 1 .. 4 q + 2, so that each value's partial sum
+    // (value % 4) is known at compile time
+#pragma unroll 1
+    for (int q = 0; q < kGroupsPerImage / 4; ++q) {
+#pragma unroll
+      for (int o = 0; o < 4; ++o) {
+        if (o % kGroups == 0 && !mbar_wait(&sm.full[slot], phase, abort_flag)) goto fail;
+        const Tin* rows =
+            reinterpret_cast<const Tin*>(sm.ring[slot] + (o % kGroups) * 4 * kRowBytes);
+        float b = compress_group(rows, jc, o == 3 && q == kGroupsPerImage / 4 - 1, carry);
+        if (o % kGroups == kGroups - 1) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.empty[slot]);
+          if (++slot == kNumStages) {
+            slot = 0;
+            phase ^= 1u;
           }
         }
-        const uint32_t within = static_cast<uint32_t>(i0 % kR);
-        const uint32_t chunk = gc0 + static_cast<uint32_t>(i0 / kR);
-        const uint32_t buf = chunk & 1;
-        if (within == 0 &&
-            !mbar_wait(&sm.a_empty[buf], ((chunk >> 1) & 1u) ^ 1u, abort_flag))
-          goto fail;
-        if constexpr (kDct == 1) {
-          const uint4 w = make_uint4(to_tf32(b[0]), to_tf32(b[1]), to_tf32(b[2]), to_tf32(b[3]));
-          *reinterpret_cast<uint4*>(sm.ops[buf] + sw128_offset(j, within, 4)) = w;
-        } else {
-          uint32_t h01, l01, h23, l23;
-          split_bf16x2(b[0], b[1], h01, l01);
-          split_bf16x2(b[2], b[3], h23, l23);
-          const uint32_t off = sw64_offset(j, within, 2);
-          *reinterpret_cast<uint2*>(sm.ops[buf] + off) = make_uint2(h01, h23);
-          *reinterpret_cast<uint2*>(sm.ops[buf] + DctTraits<kDct>::kALo + off) = make_uint2(l01, l23);
-        }
-        if (within + 4 == static_cast<uint32_t>(kR)) {
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.a_full[buf]);
-        }
-      }
-      if constexpr (!kRgb) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.empty[(g0 + 127) % kNumStages]);
-      }
-      {
-        const uint32_t acc = it & 1;
-        if (!mbar_wait(&sm.acc_full[acc], (it >> 1) & 1u, abort_flag)) goto fail;
-        tc_fence_after();
-        uint32_t tr[16];
-        tmem_ld16_nowait(sm.tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + acc * 16, tr);
-        tmem_ld_wait();
-        tmem_take16(tr);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
-        if (active) {
+        const int i = 4 * q + o - 1;
+        if (o == 0 && q == 0) b = 0.0f;  // there is no value -1
+        if (buf1 && i >= 0) buf1[i * 128] = b;
+        if constexpr (kDct == 0) {
+          const float4* d4 = reinterpret_cast<const float4*>(sm.dt[i + 1]);
+          const float2 bb = make_float2(b, b);
 #pragma unroll
-          for (int k = 0; k < 16; ++k) sm.t[k][j] = __uint_as_float(tr[k]);
+          for (int k = 0; k < 4; ++k) {
+            const float4 d = d4[k];
+            float2& a0 = acc[2 * k][(o + 3) & 3];
+            float2& a1 = acc[2 * k + 1][(o + 3) & 3];
+            a0 = add2_rn(a0, mul2_rn(make_float2(d.x, d.y), bb, nz));
+            a1 = add2_rn(a1, mul2_rn(make_float2(d.z, d.w), bb, nz));
+          }
+        } else {
+          unit[(o + 3) & 3] = active ? b : 0.0f;
+          if (o == 0 && q > 0 && !write_unit(q - 1)) goto fail;
+        }
+      }
+    }
+    if constexpr (kDct == 0) {
+      if (active) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float2 t = add2_rn(add2_rn(add2_rn(acc[k][0], acc[k][1]), acc[k][2]), acc[k][3]);
+          sm.t[2 * k][j] = t.x;
+          sm.t[2 * k + 1][j] = t.y;
         }
       }
     } else {
-    float acc[16][4];
-
-#pragma unroll
-    for (int k = 0; k < 16; ++k)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[k][r] = 0.0f;
-
-    if (!mbar_wait(&sm.full[g0 % kNumStages], (g0 / kNumStages) & 1u, abort_flag)) goto fail;
-    if constexpr (kRgb) {
-      convert_stage_warp<Tin>(sm.ring[g0 % kNumStages], sm.conv[warp][g0 % 3], warp, lane);
+      unit[3] = 0.0f;  // value 127
+      if (!write_unit(kGroupsPerImage / 4 - 1)) goto fail;
+      const uint32_t ac = it & 1;
+      if (!mbar_wait(&sm.acc_full[ac], (it >> 1) & 1u, abort_flag)) goto fail;
+      tc_fence_after();
+      uint32_t tr[16];
+      tmem_ld16_nowait(sm.tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + ac * 16, tr);
+      tmem_ld_wait();
+      tmem_take16(tr);
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.empty[g0 % kNumStages]);
-    }
-    HCarry hc{};
-    CompressCarry cc{};
-    if (kSep && active)
-      hcarry_init<CT, kCRow>(stage_ptr<Tin, CT, kNumStages>(sm, g0, warp), jc, hc);
-    for (int i0 = 0; i0 < 128; i0 += 4) {
+      if (lane == 0) mbar_arrive(&sm.acc_empty[ac]);
+      if (active) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int i = i0 + r;
-        if (i < 127) {
-          const uint32_t ga = g0 + i, gb = ga + 1;
-          if (!mbar_wait(&sm.full[gb % kNumStages], (gb / kNumStages) & 1u, abort_flag))
-            goto fail;
-          if constexpr (kRgb) {
-            convert_stage_warp<Tin>(sm.ring[gb % kNumStages], sm.conv[warp][gb % 3], warp, lane);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.empty[gb % kNumStages]);
-          }
-          float b = 0.0f;
-          if (active) {
-            const CT* st0 = stage_ptr<Tin, CT, kNumStages>(sm, ga, warp);
-            const CT* st1 = stage_ptr<Tin, CT, kNumStages>(sm, gb, warp);
-            b = kSep ? compress_separable<CT, kCRow>(st1, jc, hc)
-                     : compress_next<CT, kCRow>(st0, st1, jc, i == 0, cc);
-            if (prm.buf1) prm.buf1[(n * 127 + i) * 128 + j] = b;
-          }
-          const float4* d4 = reinterpret_cast<const float4*>(&sm.dt[i][0]);
-          const float4 da = d4[0], db = d4[1], dc = d4[2], dd = d4[3];
-          const float d[16] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w,
-                               dc.x, dc.y, dc.z, dc.w, dd.x, dd.y, dd.z, dd.w};
-#pragma unroll
-          for (int k = 0; k < 16; ++k) acc[k][r] = __fadd_rn(acc[k][r], __fmul_rn(d[k], b));
-          if constexpr (!kRgb) {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.empty[ga % kNumStages]);
-          }
-        }
+        for (int k = 0; k < 16; ++k) sm.t[k][j] = __uint_as_float(tr[k]);
       }
     }
-    if constexpr (!kRgb) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.empty[(g0 + 127) % kNumStages]);
-    }
-
-    if (active) {
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        sm.t[k][j] = __fadd_rn(__fadd_rn(__fadd_rn(acc[k][0], acc[k][1]), acc[k][2]), acc[k][3]);
-    }
-    }  // FP32 stage 1
     named_bar_sync(kComputeBarrier, kComputeThreads);
     {
       // stage 2: P[k][c] = sum_m T[k][m] * D[c][m]; thread -> (k, c0), (k, c0 + 1)
       const int k = tid >> 3, c0 = (tid & 7) * 2;
-      float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+      float2 sum[4] = {};
+#pragma unroll 8
       for (int m0 = 0; m0 < 128; m0 += 4) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const int m = m0 + r;
           if (m < 127) {
             const float tv = sm.t[k][m];
-            s0[r] = __fadd_rn(s0[r], __fmul_rn(tv, sm.dr[c0][m]));
-            s1[r] = __fadd_rn(s1[r], __fmul_rn(tv, sm.dr[c0 + 1][m]));
+            const float2 d = *reinterpret_cast<const float2*>(&sm.dt[m + 1][c0]);
+            sum[r] = add2_rn(sum[r], mul2_rn(d, make_float2(tv, tv), nz));
           }
         }
       }
-      const float o0 = __fadd_rn(__fadd_rn(__fadd_rn(s0[0], s0[1]), s0[2]), s0[3]);
-      const float o1 = __fadd_rn(__fadd_rn(__fadd_rn(s1[0], s1[1]), s1[2]), s1[3]);
+      const float2 p = add2_rn(add2_rn(add2_rn(sum[0], sum[1]), sum[2]), sum[3]);
       const int pb = it & 1;
       if (!mbar_wait(&sm.pempty[pb], ((it >> 1) & 1u) ^ 1u, abort_flag)) goto fail;
-      sm.p[pb][k * 16 + c0] = o0;
-      sm.p[pb][k * 16 + c0 + 1] = o1;
+      *reinterpret_cast<float2*>(&sm.p[pb][k * 16 + c0]) = p;
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.pfull[pb]);
     }
@@ -1057,8 +966,8 @@ fail:
 // Bound by the latency of that sequence: of ~12,500 clk for one f32 image, ~2,800 until the
 // rows are there, ~2,000 compress (8 conflict-free 16-byte loads per value), ~500 for each of
 // the two exchanges, ~1,150 per DCT stage and ~4,200 epilogue (2,150 of them the gradient
-// sum). Back to back, one image: 8.5 us (hash_kernel 40.6; RGB8 10.4, was 77); 37 u8 images
-// 14.6 us (43.2); 64 f32 images 32 us (41.3).
+// sum). Back to back, one image: 8.5 us (hash_kernel 31 us for f32, 29 u8); RGB8 10.4 us (41);
+// 37 u8 images 14.5 us (29); 56 f32 images 27.3 us (31).
 constexpr int kSplitCtas = 8;        // CTAs per image (the portable cluster size)
 constexpr int kSplitThreads = 512;
 constexpr int kSplitRows = 128 / kSplitCtas;           // compressed rows per CTA
@@ -1357,12 +1266,14 @@ __global__ void __cluster_dims__(kSplitCtas, 1, 1) __launch_bounds__(kSplitThrea
   float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   const int i0 = kSplitRows * rank + 4 * g;
   if (j < 127) {
-    CompressCarry cc{};
+    // the group before the first value starts it; group r + 1 finishes value r
+    const Tin* st = reinterpret_cast<const Tin*>(rows + 16 * g * kRowBytes);
+    TapSum carry;
+    compress_group(st, j, false, carry);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (i0 + r < 127) {
-        const Tin* st = reinterpret_cast<const Tin*>(rows + (4 * (4 * g + r)) * kRowBytes);
-        b[r] = compress_next<Tin>(st, st + 4 * 512, j, r == 0, cc);
+        b[r] = compress_group(st + 4 * (r + 1) * 512, j, r == 3 || i0 + r == 126, carry);
         if (prm.buf1) prm.buf1[(n * 127 + i0 + r) * 128 + j] = b[r];
       }
     }
@@ -1439,8 +1350,8 @@ __global__ void __launch_bounds__(128) dihedral_kernel(const DihedralLaunch prm)
 
 template <typename Tin, int kDct>
 static size_t hash_smem_bytes() {
-  return sizeof(HashSmem<4 * InputTraits<Tin>::kRowBytes, ring_stages<Tin, kDct>(), kDct,
-                         conv_slots<Tin>()>) +
+  return sizeof(HashSmem<4 * stage_groups<Tin>() * InputTraits<Tin>::kRowBytes,
+                         ring_stages<Tin, kDct>(), kDct>) +
          1024;  // + base alignment
 }
 
@@ -1548,25 +1459,22 @@ static cudaError_t set_split_smem() {
                               static_cast<int>(split_smem_bytes<Tin>()));
 }
 template <typename Tin>
-static cudaError_t launch_split(HashLaunch p, cudaStream_t s) {
-  p.neg_zero = -0.0f;
+static cudaError_t launch_split(const HashLaunch& p, cudaStream_t s) {
   hash_split_kernel<Tin><<<static_cast<unsigned>(kSplitCtas * p.n), kSplitThreads,
                            split_smem_bytes<Tin>(), s>>>(p);
   return cudaGetLastError();
 }
 
 // Largest batch that hash_split_kernel takes. Its time grows with the waves of clusters (16 or
-// more images at once), hash_kernel's steps with the CTAs per SM: 41 us (f32, u8; RGB 80 us)
-// up to 152 images, 47-51 us (95-97 us) up to 304. Measured on both sides, split against
-// persistent: f32 39.4 / 41.3 us at 88 and 43.7 / 41.3 at 96 images; u8 46.9 / 50.7 at 208
-// and 49.6 / 50.5 at 224; RGB8 91.2 / 96.7 at 192 and 97.7 / 96.6 at 208; RGBA8 88.2 / 96.7
-// at 176 and 95.2 / 97.2 at 192.
+// more images at once), hash_kernel's is that of one image on a CTA up to 152 images (f32
+// 31-38 us, u8 29 us, RGB 41 us). Measured on both sides, split against persistent: f32
+// 27.3 / 31.1 us at 56 images and 32.0 / 31.4 at 64; u8 26.9 / 29.0 at 104 and 28.9 / 29.0 at
+// 112; RGB8 36.2 / 41.2 at 72 and 41.8 / 41.2 at 80; RGBA8 38.0 / 41.2 and 43.5 / 41.2.
 static int64_t split_max_images(int input_kind) {
   switch (input_kind) {
-    case YPDQ_INPUT_F32: return 88;
-    case YPDQ_INPUT_U8: return 208;
-    case YPDQ_INPUT_RGB8: return 184;
-    default: return 176;
+    case YPDQ_INPUT_F32: return 56;
+    case YPDQ_INPUT_U8: return 104;
+    default: return 72;
   }
 }
 
@@ -1574,8 +1482,10 @@ cudaError_t hash_occupancy_variant(int input_kind, int dct, int separable, int* 
   return dispatch<OccupancyOf>(input_kind, dct, separable, ctas_per_sm);
 }
 
-cudaError_t launch_hash(const HashLaunch& p, int num_sms, int ctas_per_sm, cudaStream_t s) {
-  if (p.n <= 0) return cudaSuccess;
+cudaError_t launch_hash(const HashLaunch& prm, int num_sms, int ctas_per_sm, cudaStream_t s) {
+  if (prm.n <= 0) return cudaSuccess;
+  HashLaunch p = prm;
+  p.neg_zero = -0.0f;
   if (p.dct == 0 && !p.separable && p.n <= split_max_images(p.input_kind)) {
     switch (p.input_kind) {
       case YPDQ_INPUT_F32: return launch_split<float>(p, s);
