@@ -113,13 +113,11 @@ void set_last_error_text(const char* text) { g_last_error = text; }
 
 namespace {
 
-// YPDQ_COMPRESS_JAROSZ: the filter passes need two f32 planes per image in flight, in a
-// context-owned scratch for chunks of up to 2,048 images (4 GiB). Each pass runs one thread
-// per line, 512 per image, so a chunk is about nine rounds of the GPU's resident warps and
-// the last, partly filled round costs little. Calls on different streams take turns on it
-// (under ctx->mu): each waits for the previous user's completion event (jarosz_done) and
-// records its own.
-int64_t jarosz_chunk(int64_t n) { return n < 2048 ? (n > 0 ? n : 1) : 2048; }
+// YPDQ_COMPRESS_JAROSZ needs a context-owned scratch: each image's PDQF (1 KiB) for chunks of
+// up to 16,384 images, and two f32 planes per image for the few images that take the planes
+// (62 MiB). Calls on different streams take turns on it (under ctx->mu): each waits for the
+// previous user's completion event (jarosz_done) and records its own.
+int64_t jarosz_chunk(int64_t n) { return n < 16384 ? (n > 0 ? n : 1) : 16384; }
 
 // Chunk bounds for ypdq_screen_host. The copy of chunk c+1 (copy stream) runs while chunk c
 // is hashed and scanned (compute stream). The copies run back to back, so with u the copy
@@ -167,9 +165,9 @@ ChunkCost screen_chunk_cost(int input_kind, bool jarosz, uint64_t n_rows, uint32
   // 256 bits; 8 queries per image
   const double pairs_per_us = threshold <= 36 ? 21.5e6 : threshold <= 62 ? 9.5e6 : 8.3e6;
   const double scan_us = 8.0 * static_cast<double>(n_rows) / pairs_per_us;
-  // the Jarosz filter: four passes, each at least one line's sequential replay (512
-  // dependent steps, ~5 us) however few images the chunk holds, plus the DCT
-  if (jarosz) return {30.0, (input_kind == YPDQ_INPUT_U8 ? 0.95 : 1.1) + scan_us};
+  // the Jarosz filter: one CTA walks an image in 80-110 us however few the images, and three
+  // CTAs share an SM
+  if (jarosz) return {80.0, (input_kind == YPDQ_INPUT_U8 ? 0.28 : 0.37) + scan_us};
   // hash_kernel runs one image per CTA, two CTAs per SM: a chunk of up to 304 images takes
   // one image's time on a CTA, 304 x the per-image rate
   const double hash_us = input_kind == YPDQ_INPUT_U8 ? 0.135 : input_kind == YPDQ_INPUT_F32 ? 0.18 : 0.28;

@@ -144,81 +144,6 @@ template <>
 struct InputTraits<rgba8_t> {
   static constexpr int kRowBytes = 512 * 4;
 };
-// Two f32 operations in one instruction, each rounded by itself. ptxas (13.0) contracts a
-// packed multiply and the packed add that takes its result into one fused operation, .rn or
-// not (scalar mul.rn / add.rn it leaves alone), which would change bits. So a product is
-// taken as fma(a, b, -0) with the -0 read from the launch parameters, a value that the
-// compiler does not know: RN(a b + -0) is RN(a b), signed zeros included, and an fma cannot
-// be contracted with a later add.
-__device__ __forceinline__ float2 fma2_rn(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "mov.b64 w, {%6, %7};\n\tfma.rn.f32x2 z, x, y, w;\n\tmov.b64 {%0, %1}, z;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b, float neg_zero) {
-  return fma2_rn(a, b, make_float2(neg_zero, neg_zero));
-}
-// The plain packed multiply, for products that only scalar adds take.
-__device__ __forceinline__ float2 mul2_contractible_rn(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "mul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-
-// Byte k (0..3) of w as the float 2^23 + byte, placed in the mantissa by a byte permute. A
-// product with a weight takes the 2^23 off again in its own rounding: RN(W byte) is
-// fma(W, 2^23 + byte, -2^23 W), one instruction for the conversion and the product, exact
-// before the rounding because 2^23 W is (no I2F on the quarter-rate pipe either).
-constexpr float kByteBias = 8388608.0f;
-template <int k>
-__device__ __forceinline__ float byte_biased(uint32_t w) {
-  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 | k));
-}
-template <int k>
-__device__ __forceinline__ float byte_f(uint32_t w) {
-  return byte_biased<k>(w) - kByteBias;
-}
-// ITU-R BT.601 luma in the reference's scalar order (Kernel::cvt_rgb8_to_luma8f,
-// src/kernel/mod.rs:303-340, coefficients src/kernel/constants.rs:23):
-// (0.299 r + 0.587 g) + 0.114 b, each product and sum rounded to f32, no fused multiply-add.
-// Two pixels at once, from biased bytes.
-__device__ __forceinline__ float2 luma2_bt601(float2 r, float2 g, float2 b) {
-  constexpr float cr = 0.299f, cg = 0.587f, cb = 0.114f;
-  const float2 pr = fma2_rn(r, make_float2(cr, cr), make_float2(-kByteBias * cr, -kByteBias * cr));
-  const float2 pg = fma2_rn(g, make_float2(cg, cg), make_float2(-kByteBias * cg, -kByteBias * cg));
-  const float2 pb = fma2_rn(b, make_float2(cb, cb), make_float2(-kByteBias * cb, -kByteBias * cb));
-  return add2_rn(add2_rn(pr, pg), pb);
-}
-// Pixels 0-1 and 2-3 of four: RGB8 in three words (r g b r | g b r g | b r g b), RGBA8 in four.
-__device__ __forceinline__ float2 luma01(uint32_t a, uint32_t b, uint32_t) {
-  return luma2_bt601(make_float2(byte_biased<0>(a), byte_biased<3>(a)),
-                     make_float2(byte_biased<1>(a), byte_biased<0>(b)),
-                     make_float2(byte_biased<2>(a), byte_biased<1>(b)));
-}
-__device__ __forceinline__ float2 luma23(uint32_t, uint32_t b, uint32_t c) {
-  return luma2_bt601(make_float2(byte_biased<2>(b), byte_biased<1>(c)),
-                     make_float2(byte_biased<3>(b), byte_biased<2>(c)),
-                     make_float2(byte_biased<0>(c), byte_biased<3>(c)));
-}
-__device__ __forceinline__ float2 luma_rgba(uint32_t p, uint32_t q) {
-  return luma2_bt601(make_float2(byte_biased<0>(p), byte_biased<0>(q)),
-                     make_float2(byte_biased<1>(p), byte_biased<1>(q)),
-                     make_float2(byte_biased<2>(p), byte_biased<2>(q)));
-}
 // The five columns 4j + 2 .. 4j + 6 of one input row in shared memory that compressed column
 // j reads: two pairs and one. f32 input and luma as they are, u8 biased (byte_biased).
 struct RowX {

@@ -76,7 +76,7 @@ struct Slot {
   uint8_t* d_hashes = nullptr;
   float* d_quality = nullptr;
   ypdq_hit* d_hits = nullptr;
-  void* d_jarosz = nullptr;  // YPDQ_COMPRESS_JAROSZ: the filter planes of a whole step
+  void* d_jarosz = nullptr;  // YPDQ_COMPRESS_JAROSZ: the scratch of a whole step
   StepHeader* d_hdr = nullptr;
   StepHeader* h_hdr = nullptr;  // pinned
   ypdq_hit* h_hits = nullptr;   // pinned, step_hit_capacity entries
