@@ -235,6 +235,15 @@ ypdq_status ypdq_ctx_create(int device, ypdq_ctx** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->jarosz_done, cudaEventDisableTiming);
+  if (e == cudaSuccess) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = ypdq_ctx::kPoolKeep;
+    e = cudaMemPoolCreate(&ctx->pool, &props);
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
   for (int i = 0; i < ypdq_ctx::kMaxChunks && e == cudaSuccess; ++i)
     e = cudaEventCreateWithFlags(&ctx->chunk_copied[i], cudaEventDisableTiming);
   if (e != cudaSuccess) {
@@ -261,6 +270,7 @@ ypdq_status ypdq_ctx_destroy(ypdq_ctx* ctx) {
   if (ctx->jarosz_scratch) cudaFree(ctx->jarosz_scratch);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   if (ctx->jarosz_done) cudaEventDestroy(ctx->jarosz_done);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->d_err) cudaFree(ctx->d_err);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
@@ -479,7 +489,7 @@ ypdq_status ypdq_sort_hits(ypdq_ctx* ctx, ypdq_hit* d_hits, uint64_t n, ypdq_str
   ypdq_status st = check_ctx(ctx);
   if (st) return st;
   if (n > 0 && !d_hits) return fail(YPDQ_ERR_INVALID, "d_hits is NULL");
-  CK(launch_sort_hits(d_hits, n, reinterpret_cast<cudaStream_t>(stream)), "sort launch");
+  CK(launch_sort_hits(d_hits, n, ctx->pool, reinterpret_cast<cudaStream_t>(stream)), "sort launch");
   return YPDQ_OK;
 }
 
@@ -614,7 +624,7 @@ ypdq_status ypdq_screen_host(ypdq_ctx* ctx, ypdq_db* db, const void* h_images, i
   uint64_t total = 0;
   memcpy(&total, stage, sizeof(total));
   const uint64_t m = total < capacity ? total : capacity;
-  CK(launch_sort_hits(static_cast<ypdq_hit*>(d_hits), m, s), "sort launch");
+  CK(launch_sort_hits(static_cast<ypdq_hit*>(d_hits), m, ctx->pool, s), "sort launch");
   if (m > 0) CK(cudaMemcpyAsync(stage + 64, d_hits, m * sizeof(ypdq_hit), cudaMemcpyDeviceToHost, s), "D2H hits");
   if (h_hashes && n > 0) CK(cudaMemcpyAsync(h_hashes, d_hash, 256 * n, cudaMemcpyDeviceToHost, s), "D2H hashes");
   if (h_quality && n > 0) CK(cudaMemcpyAsync(h_quality, d_q, 32 * n, cudaMemcpyDeviceToHost, s), "D2H quality");

@@ -30,6 +30,10 @@ struct ypdq_ctx {
   void* jarosz_scratch = nullptr;  // YPDQ_COMPRESS_JAROSZ filter planes
   size_t jarosz_bytes = 0;
   cudaEvent_t jarosz_done = nullptr;  // recorded after the last work that used it
+  // stream-ordered temporaries (the hit sort's second buffer); keeps at most kPoolKeep bytes
+  // between calls
+  cudaMemPool_t pool = nullptr;
+  static constexpr uint64_t kPoolKeep = 64ull << 20;
 };
 
 struct ypdq_db {

@@ -9,6 +9,8 @@
 //   SIMT   one row per thread, eight 32-bit XOR + POPC per (row, query);
 //   B1MMA  16 rows x 8 queries per warp instruction with the binary tensor-core MMA
 //          (mma.sync m16n8k256 .b1 .xor.popc), whose accumulator is the distance.
+#include <cstddef>
+
 #include "ypdq_internal.cuh"
 
 namespace ypdq {
@@ -247,6 +249,8 @@ __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
+cudaError_t sort_init();
+
 cudaError_t scan_init() {
   const int smem = static_cast<int>(kMaxSmemQueries * 32);
   cudaError_t e = cudaSuccess;
@@ -257,6 +261,8 @@ cudaError_t scan_init() {
     if (e != cudaSuccess) return e;
   }
   e = cudaFuncSetAttribute(scan_b1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  e = sort_init();
   if (e != cudaSuccess) return e;
   return scan_tc_init();
 }
@@ -332,8 +338,240 @@ cudaError_t launch_scan(const ScanLaunch& p, int algo, int num_sms, cudaStream_t
 }
 
 // ---------------------------------------------------------------- hit sorting
+//
+// By (index, query), the scalar matcher's visit order, through a second buffer: few hits by
+// counting for each the hits before it, more by a merge sort (tiles sorted in shared memory,
+// then passes that merge runs in pairs).
 
-// Order by (index, query): the scalar matcher's visit order.
+// A hit as two words: the index, and query | distance << 32.
+struct Hit2 {
+  uint64_t k, v;
+};
+static_assert(sizeof(Hit2) == sizeof(ypdq_hit) && offsetof(ypdq_hit, query) == 8 &&
+                  offsetof(ypdq_hit, distance) == 12,
+              "a hit is its index and query | distance << 32");
+__device__ __forceinline__ bool less2(const Hit2& a, const Hit2& b) {
+  return a.k < b.k || (a.k == b.k && static_cast<uint32_t>(a.v) < static_cast<uint32_t>(b.v));
+}
+__device__ __forceinline__ Hit2 load_hit(const ypdq_hit* h, uint64_t i) {  // 8-byte aligned
+  const uint64_t* p = reinterpret_cast<const uint64_t*>(h + i);
+  return {p[0], p[1]};
+}
+__device__ __forceinline__ void store_hit(ypdq_hit* h, uint64_t i, const Hit2& x) {
+  uint64_t* p = reinterpret_cast<uint64_t*>(h + i);
+  p[0] = x.k;
+  p[1] = x.v;
+}
+
+// Whether the hit with keys y (index; query, then position) comes before one with k and s.
+__device__ __forceinline__ uint32_t is_before(uint64_t yk, uint64_t ys, uint64_t k, uint64_t s) {
+  return yk < k || (yk == k && ys < s) ? 1u : 0u;
+}
+
+// Rank of each hit among all n (of equal ones the first first), and the hit to its place.
+// Block: 32 hits, one per lane; its warps share the comparisons with all n, every lane of a
+// warp with the same hit at a time (a broadcast load from cache; 32 hits at a time through
+// shared memory with two hits per lane was slower, 70 against 45 us for 8,192). Quadratic, but
+// one launch over the whole chip.
+constexpr int kRankWarps = 16;
+__global__ void __launch_bounds__(32 * kRankWarps)
+    rank_hits_kernel(const ypdq_hit* __restrict__ in, ypdq_hit* __restrict__ out, uint32_t n) {
+  __shared__ uint32_t before[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = 32 * blockIdx.x + lane;
+  if (warp == 0) before[lane] = 0;
+  __syncthreads();
+  const Hit2 x = load_hit(in, min(i, n - 1));
+  const uint64_t xs = (x.v << 32) | i;
+  const uint32_t each = (n + kRankWarps - 1) / kRankWarps, first = warp * each;
+  const uint32_t end = min(first + each, n);
+  uint32_t c = 0;
+#pragma unroll 8
+  for (uint32_t j = first; j < end; ++j) {
+    const Hit2 y = load_hit(in, j);
+    c += is_before(y.k, (y.v << 32) | j, x.k, xs);
+  }
+  atomicAdd(&before[lane], c);
+  __syncthreads();
+  if (warp == 0 && i < n) store_hit(out, before[lane], x);
+}
+
+// The same in place for one block's worth of hits.
+constexpr int kSmallSort = 256;
+__global__ void __launch_bounds__(kSmallSort) rank_small_kernel(ypdq_hit* h, uint32_t n) {
+  __shared__ ulonglong2 all[kSmallSort];
+  const uint32_t i = threadIdx.x;
+  Hit2 x{};
+  if (i < n) {
+    x = load_hit(h, i);
+    all[i] = make_ulonglong2(x.k, (x.v << 32) | i);
+  }
+  __syncthreads();
+  if (i >= n) return;
+  const uint64_t xs = (x.v << 32) | i;
+  uint32_t c = 0;
+#pragma unroll 8
+  for (uint32_t j = 0; j < n; ++j) {
+    const ulonglong2 y = all[j];
+    c += is_before(y.x, y.y, x.k, xs);
+  }
+  store_hit(h, c, x);
+}
+
+constexpr int kSortItems = 8;  // hits per thread
+// Place of item i in a shared tile: one hit of padding after every eight, so that threads
+// reading eight consecutive hits each (16 bytes at a time) meet different banks.
+__host__ __device__ constexpr int padded(int i) { return i + i / kSortItems; }
+__device__ __forceinline__ ulonglong2& slot_of(Hit2* sh, int i) {
+  return *reinterpret_cast<ulonglong2*>(sh + padded(i));
+}
+__device__ __forceinline__ Hit2 get(Hit2* sh, int i) {
+  const ulonglong2 x = slot_of(sh, i);
+  return {x.x, x.y};
+}
+__device__ __forceinline__ void put(Hit2* sh, int i, const Hit2& h) {
+  slot_of(sh, i) = make_ulonglong2(h.k, h.v);
+}
+
+// The kSortItems outputs from position d on of merging sh[a .. a + na) and sh[b .. b + nb)
+// (each sorted; equal hits from the first run first) into out. Items past the end are whatever
+// lies there: the caller drops them.
+__device__ __forceinline__ void merge_items(Hit2* sh, int a, int na, int b, int nb, int d,
+                                            Hit2 (&out)[kSortItems]) {
+  int lo = d > nb ? d - nb : 0, hi = d < na ? d : na;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (!less2(get(sh, b + d - 1 - mid), get(sh, a + mid))) lo = mid + 1;
+    else hi = mid;
+  }
+  int i = lo, j = d - lo;
+  // the item a run offers next; past its end (or of an empty run) any item of the tile
+  const auto of_a = [&](int at) { return get(sh, na > 0 ? a + min(at, na - 1) : b); };
+  const auto of_b = [&](int at) { return get(sh, nb > 0 ? b + min(at, nb - 1) : a); };
+  Hit2 x = of_a(i), y = of_b(j);
+#pragma unroll
+  for (int q = 0; q < kSortItems; ++q) {
+    const bool first = j >= nb || (i < na && !less2(y, x));
+    out[q] = first ? x : y;
+    i += first ? 1 : 0;
+    j += first ? 0 : 1;
+    const Hit2 z = first ? of_a(i) : of_b(j);
+    if (first) x = z;
+    else y = z;
+  }
+}
+
+// Tile blockIdx.x of kThreads * 8 hits: eight sorted in each thread's registers, then merged
+// in pairs of runs through shared memory. Positions past n hold +infinity.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) sort_tiles_kernel(const ypdq_hit* in, ypdq_hit* out,
+                                                              uint64_t n) {
+  constexpr int kTile = kThreads * kSortItems;
+  extern __shared__ __align__(16) uint8_t sort_smem[];
+  Hit2* sh = reinterpret_cast<Hit2*>(sort_smem);
+  const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kTile;
+  const int count = static_cast<int>(n - base < kTile ? n - base : kTile);
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < kSortItems; ++q) {
+    const int i = q * kThreads + tid;
+    put(sh, i, i < count ? load_hit(in, base + i) : Hit2{~0ull, ~0ull});
+  }
+  __syncthreads();
+  Hit2 x[kSortItems];
+#pragma unroll
+  for (int q = 0; q < kSortItems; ++q) x[q] = get(sh, tid * kSortItems + q);
+  // odd-even transposition: 8 rounds sort 8 items
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r)
+#pragma unroll
+    for (int q = r & 1; q + 1 < kSortItems; q += 2)
+      if (less2(x[q + 1], x[q])) {
+        const Hit2 t = x[q];
+        x[q] = x[q + 1];
+        x[q + 1] = t;
+      }
+#pragma unroll
+  for (int q = 0; q < kSortItems; ++q) put(sh, tid * kSortItems + q, x[q]);
+  __syncthreads();
+  for (int w = kSortItems; w < count; w <<= 1) {
+    const int at = tid * kSortItems, first = at / (2 * w) * (2 * w);
+    merge_items(sh, first, w, first + w, w, at - first, x);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kSortItems; ++q) put(sh, at + q, x[q]);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int q = 0; q < kSortItems; ++q) {
+    const int i = q * kThreads + tid;
+    if (i < count) store_hit(out, base + i, get(sh, i));
+  }
+}
+
+// How many of the first d outputs of merging runs a (na hits) and b (nb) come from a: the
+// merge path's crossing of diagonal d, by one warp with 32 probes at a time.
+__device__ __forceinline__ uint64_t merge_path_warp(const ypdq_hit* a, uint64_t na,
+                                                    const ypdq_hit* b, uint64_t nb, uint64_t d,
+                                                    int lane) {
+  uint64_t lo = d > nb ? d - nb : 0, hi = d < na ? d : na;
+  while (lo < hi) {
+    const uint64_t span = hi - lo;
+    const uint64_t mid = span <= 32 ? lo + lane : lo + span * (lane + 1) / 33;
+    const bool right = mid < hi && !less2(load_hit(b, d - 1 - mid), load_hit(a, mid));
+    const int c = __popc(__ballot_sync(0xffffffffu, right));  // true for a prefix of the lanes
+    if (span <= 32) return lo + c;
+    const uint64_t next_lo = c > 0 ? __shfl_sync(0xffffffffu, mid, c > 0 ? c - 1 : 0) + 1 : lo;
+    const uint64_t next_hi = c < 32 ? __shfl_sync(0xffffffffu, mid, c < 32 ? c : 31) : hi;
+    lo = next_lo;
+    hi = next_hi;
+  }
+  return lo;
+}
+
+// One pass: runs of w hits (a multiple of the block's 2,048 outputs) merged in pairs.
+constexpr int kMergeThreads = 256;
+constexpr int kMergeTile = kMergeThreads * kSortItems;
+__global__ void __launch_bounds__(kMergeThreads)
+    merge_runs_kernel(const ypdq_hit* in, ypdq_hit* out, uint64_t n, uint64_t w) {
+  __shared__ __align__(16) Hit2 sh[padded(kMergeTile)];
+  __shared__ uint64_t cut[2];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint64_t o = static_cast<uint64_t>(blockIdx.x) * kMergeTile;
+  const uint64_t first = o / (2 * w) * (2 * w);
+  const uint64_t na = n - first < w ? n - first : w;
+  const uint64_t nb = n - first - na < w ? n - first - na : w;
+  const ypdq_hit* a = in + first;
+  const ypdq_hit* b = a + na;
+  const uint64_t d0 = o - first, d1 = d0 + kMergeTile < na + nb ? d0 + kMergeTile : na + nb;
+  if (warp < 2) {
+    const uint64_t c = merge_path_warp(a, na, b, nb, warp == 0 ? d0 : d1, lane);
+    if (lane == 0) cut[warp] = c;
+  }
+  __syncthreads();
+  const uint64_t a0 = cut[0], b0 = d0 - a0;
+  const int ca = static_cast<int>(cut[1] - a0), count = static_cast<int>(d1 - d0);
+#pragma unroll
+  for (int q = 0; q < kSortItems; ++q) {
+    const int i = q * kMergeThreads + tid;
+    if (i < count) put(sh, i, i < ca ? load_hit(a, a0 + i) : load_hit(b, b0 + (i - ca)));
+  }
+  __syncthreads();
+  Hit2 x[kSortItems];
+  const int at = tid * kSortItems;
+  if (at < count) merge_items(sh, 0, ca, ca, count - ca, at, x);
+  __syncthreads();
+  if (at < count)
+#pragma unroll
+    for (int q = 0; q < kSortItems; ++q) put(sh, at + q, x[q]);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kSortItems; ++q) {
+    const int i = q * kMergeThreads + tid;
+    if (i < count) store_hit(out, o + i, get(sh, i));
+  }
+}
+
+// The bitonic sort in place. Order by (index, query): the scalar matcher's visit order.
 __device__ __forceinline__ bool hit_less(const ypdq_hit& a, const ypdq_hit& b) {
   return a.index < b.index || (a.index == b.index && a.query < b.query);
 }
@@ -401,8 +639,7 @@ __global__ void __launch_bounds__(kSortBlock / 2)
     if (base + x < n) h[base + x] = sh[x];
 }
 
-cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaStream_t s) {
-  if (n < 2) return cudaSuccess;
+static cudaError_t launch_sort_in_place(ypdq_hit* hits, uint64_t n, cudaStream_t s) {
   uint64_t padded = 1;
   while (padded < n) padded <<= 1;
   const unsigned threads = 256;
@@ -419,6 +656,63 @@ cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaStream_t s) {
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
+}
+
+constexpr int kTileThreads = 512;
+constexpr size_t kSortSmem = sizeof(Hit2) * padded(kTileThreads * kSortItems);
+
+cudaError_t sort_init() {
+  return cudaFuncSetAttribute(sort_tiles_kernel<kTileThreads>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(kSortSmem));
+}
+
+// Up to 256 hits: one block, in place. Up to 8,192: rank_hits_kernel (45 us there, event-timed
+// with its launches, against 64 for one tile and 60 for two tiles and a pass just above; at
+// 10,000 hits 67 against 60). Past that the merge sort. The bitonic sort that did all of this
+// before, in place with every step wider than 2,048 hits a launch of its own, took 23 us for
+// 100 hits (now 11), 39 for 1,000 (18), 85 for 8,192 (45), 107 for 10,000 (60), 200 for 100,000
+// (91) and 751 for 1.02 M (184); it stays for the case that the second buffer cannot be had.
+// Tiles of 4,096 hits: 2,048 and 8,192 take 190 and 177 us for 1.02 M but 63 and 73 for 10,000.
+constexpr uint64_t kRankMax = 8192;
+
+cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cudaStream_t s) {
+  if (n < 2) return cudaSuccess;
+  if (n <= static_cast<uint64_t>(kSmallSort)) {
+    rank_small_kernel<<<1, kSmallSort, 0, s>>>(hits, static_cast<uint32_t>(n));
+    return cudaGetLastError();
+  }
+  void* second = nullptr;
+  if (!pool || cudaMallocFromPoolAsync(&second, n * sizeof(ypdq_hit), pool, s) != cudaSuccess) {
+    cudaGetLastError();
+    return launch_sort_in_place(hits, n, s);
+  }
+  ypdq_hit* const other = static_cast<ypdq_hit*>(second);
+  cudaError_t e = cudaSuccess;
+  if (n <= kRankMax) {
+    rank_hits_kernel<<<static_cast<unsigned>((n + 31) / 32), 32 * kRankWarps, 0, s>>>(
+        hits, other, static_cast<uint32_t>(n));
+    e = cudaMemcpyAsync(hits, other, n * sizeof(ypdq_hit), cudaMemcpyDeviceToDevice, s);
+  } else {
+    constexpr uint64_t kTile = kTileThreads * kSortItems;
+    // the tiles go where an even number of passes from there ends in `hits`
+    int passes = 0;
+    for (uint64_t w = kTile; w < n; w <<= 1) ++passes;
+    ypdq_hit* from = passes % 2 ? other : hits;
+    ypdq_hit* to = passes % 2 ? hits : other;
+    sort_tiles_kernel<kTileThreads>
+        <<<static_cast<unsigned>((n + kTile - 1) / kTile), kTileThreads, kSortSmem, s>>>(hits, from, n);
+    for (uint64_t w = kTile; w < n; w <<= 1) {
+      merge_runs_kernel<<<static_cast<unsigned>((n + kMergeTile - 1) / kMergeTile), kMergeThreads, 0, s>>>(
+          from, to, n, w);
+      ypdq_hit* t = from;
+      from = to;
+      to = t;
+    }
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  const cudaError_t f = cudaFreeAsync(second, s);
+  return e != cudaSuccess ? e : f;
 }
 
 }  // namespace ypdq
