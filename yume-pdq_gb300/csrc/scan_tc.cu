@@ -220,6 +220,7 @@ struct Params {
   uint32_t pack_offset;   // byte offset of the packed ring in shared memory
   uint32_t a_stages;      // expanded tiles in flight
   uint32_t b_offset;      // byte offset of the expanded queries
+  uint32_t queue_offset;  // byte offset of the candidate queues (t <= 36)
   uint64_t wait_ns;       // longest barrier wait before the kernel gives up (timeout flag)
   int stall;              // testing: the producer issues no copies, so the waits run out
 };
@@ -251,13 +252,12 @@ __device__ __forceinline__ uint64_t candidate_mask(const uint32_t (&raw)[32], fl
 // lane without candidates passes cand = 0. The loops run once per candidate of the lane,
 // which keeps this rare path short: it runs while the tile's epilogue warp holds up the next
 // tile, and a planted near-duplicate row makes it run for several queries of a pass.
-// (stride: bit j of cand stands for query q_first + stride * j; 1 unless given.)
 __device__ __forceinline__ void emit_candidates(uint64_t cand, uint64_t row, uint64_t q_first,
                                                 uint32_t n_queries, const Params& prm,
-                                                int lane, uint32_t stride = 1) {
+                                                int lane) {
   {
     // bits whose query is past the end
-    const uint64_t lim = q_first >= n_queries ? 0 : (n_queries - q_first + stride - 1) / stride;
+    const uint64_t lim = q_first >= n_queries ? 0 : n_queries - q_first;
     if (lim < 64) cand &= (1ull << lim) - 1;
   }
   uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
@@ -270,7 +270,7 @@ __device__ __forceinline__ void emit_candidates(uint64_t cand, uint64_t row, uin
   uint64_t hits = 0;
   for (uint64_t m = cand; m; m &= m - 1) {
     const int j = __ffsll(static_cast<long long>(m)) - 1;
-    const uint4* qp = reinterpret_cast<const uint4*>(qbase + static_cast<uint64_t>(stride) * j * 32);
+    const uint4* qp = reinterpret_cast<const uint4*>(qbase + static_cast<uint64_t>(j) * 32);
     if (popc256(r0, r1, __ldg(qp), __ldg(qp + 1)) <= prm.threshold) hits |= 1ull << j;
   }
   const uint32_t mine = static_cast<uint32_t>(__popcll(hits));
@@ -289,21 +289,85 @@ __device__ __forceinline__ void emit_candidates(uint64_t cand, uint64_t row, uin
   for (uint64_t m = hits; m; m &= m - 1, ++pos) {
     if (pos >= prm.capacity) break;
     const int j = __ffsll(static_cast<long long>(m)) - 1;
-    const uint4* qp = reinterpret_cast<const uint4*>(qbase + static_cast<uint64_t>(stride) * j * 32);
+    const uint4* qp = reinterpret_cast<const uint4*>(qbase + static_cast<uint64_t>(j) * 32);
     ypdq_hit h;
     h.index = row;
-    h.query = static_cast<uint32_t>(q_first + static_cast<uint64_t>(stride) * j) + prm.query_base;
+    h.query = static_cast<uint32_t>(q_first + j) + prm.query_base;
     h.distance = popc256(r0, r1, __ldg(qp), __ldg(qp + 1));
     prm.hits[pos] = h;
   }
 }
 
-// emit_candidates as a call: the pair kernel's epilogue reaches it only on the rare tiles with a
-// candidate, and inlined at each of its chunks it would crowd the registers of the common path.
-__device__ __noinline__ void emit_candidates_call(uint64_t cand, uint64_t row, uint64_t q_first,
-                                                  uint32_t n_queries, const Params* prm,
-                                                  int lane, uint32_t stride) {
-  emit_candidates(cand, row, q_first, n_queries, *prm, lane, stride);
+// Candidates of the scans at t <= 36, kept by each epilogue warp in shared memory and re-checked
+// a queue at a time, one candidate per lane. Re-checking them where they were found (row and
+// query loads, popcounts, an atomic: ~1.1 us for one candidate, while the tile's accumulator
+// stage and with it the SM's MMAs waited) cost a 10M-row scan with 10,000 hits 150 us where
+// one without hits took 81; with the queues and the decode by eight columns 111 and 78 (64
+// queries), 720 queries 421 -> 339, 8,192 queries 3,852 -> 3,283, 1,024 clustered queries on
+// 100M rows with 1.02 M hits 6,321 -> 5,492.
+constexpr uint32_t kQueueHits = 64;  // flushed past 32: one step of a push adds at most 32
+struct HitQueue {
+  uint64_t row[kQueueHits];
+  uint32_t query[kQueueHits];
+};
+constexpr size_t kQueueBytes = kEpilogueWarps * sizeof(HitQueue);
+
+// Re-check the first `count` candidates of the warp's queue exactly and report the hits, with
+// one atomic per 32. Called by all 32 lanes.
+__device__ __noinline__ void flush_candidates(const HitQueue* queue, uint32_t count,
+                                              const Params* prm, int lane) {
+  __syncwarp();
+  for (uint32_t at = 0; at < count; at += 32) {
+    const bool mine = at + lane < count;
+    const uint64_t row = queue->row[mine ? at + lane : at];
+    const uint32_t query = queue->query[mine ? at + lane : at];
+    const uint4* rp = reinterpret_cast<const uint4*>(prm->rows + row * 32);
+    const uint4* qp = reinterpret_cast<const uint4*>(prm->queries + static_cast<uint64_t>(query) * 32);
+    const uint32_t d = popc256(__ldg(rp), __ldg(rp + 1), __ldg(qp), __ldg(qp + 1));
+    const bool hit = mine && d <= prm->threshold;
+    const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+    if (hits == 0) continue;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(prm->count, static_cast<unsigned long long>(__popc(hits)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const uint64_t pos = base + __popc(hits & lanemask_lt());
+    if (hit && pos < prm->capacity) {
+      ypdq_hit h;
+      h.index = row;
+      h.query = query + prm->query_base;
+      h.distance = d;
+      prm->hits[pos] = h;
+    }
+  }
+  __syncwarp();
+}
+
+// Queue this lane's candidates: bit j of m is row `row + row_step * j` against query
+// `query + query_step * j` (those past the last row or query are dropped). Called by all 32
+// lanes; returns the queue's new count.
+__device__ __noinline__ uint32_t push_candidates(uint32_t m, uint64_t row, uint32_t row_step,
+                                                 uint64_t query, uint32_t query_step,
+                                                 uint32_t n_queries, HitQueue* queue,
+                                                 uint32_t count, const Params* prm, int lane) {
+  while (__any_sync(0xffffffffu, m != 0)) {
+    const int j = __ffs(static_cast<int>(m)) - 1;
+    const uint64_t r = row + static_cast<uint64_t>(row_step) * j;
+    const uint64_t q = query + static_cast<uint64_t>(query_step) * j;
+    const bool have = m != 0 && r < prm->n_rows && q < n_queries;
+    m &= m - 1;
+    const uint32_t all = __ballot_sync(0xffffffffu, have);
+    if (have) {
+      const uint32_t pos = count + __popc(all & lanemask_lt());
+      queue->row[pos] = r;
+      queue->query[pos] = static_cast<uint32_t>(q);
+    }
+    count += __popc(all);
+    if (count > kQueueHits - 32) {
+      flush_candidates(queue, count, prm, lane);
+      count = 0;
+    }
+  }
+  return count;
 }
 
 __device__ __forceinline__ void raise_abort(Smem& sm, int* dev_err) {
@@ -880,6 +944,34 @@ __device__ __forceinline__ uint32_t or_tree(const uint32_t* r) {
     return or_tree<N / 2>(r) | or_tree<N - N / 2>(r + N / 2);
 }
 
+// The rare path of a triple column's decode: one lane's candidates of eight columns, bit
+// 3 i + f for field f of column i, from v + MAGIC: its bits 7 and 15 for the first two fields,
+// and for the third the bits (a float in [2^23, 2^24), so ordered as integers) reaching
+// tc_bits. Eight columns at a time, so that those without a candidate in any lane cost only
+// their sums and a vote; masks of 64 columns at once took ~500 instructions for one candidate.
+// (v + MAGIC2, the common-case test, would keep the sums of that test in registers.)
+// Called by all 32 lanes; a lane that is not ok has none.
+__device__ __forceinline__ uint32_t triple_candidates(const uint32_t* raw, bool ok, float magic,
+                                                      uint32_t tc_bits) {
+  uint32_t r[8], m = 0, top = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    r[i] = __float_as_uint(__fadd_rn(__uint_as_float(raw[i]), magic));
+    top = max(top, r[i]);
+  }
+  const bool any = ok & ((or_tree<8>(r) & 0x8080u) != 0 || top >= tc_bits);
+  if (!__any_sync(0xffffffffu, any)) return 0;
+  if (any) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      m |= ((r[i] >> 7) & 1u) << (3 * i);
+      m |= ((r[i] >> 15) & 1u) << (3 * i + 1);
+      m |= (r[i] >= tc_bits ? 1u : 0u) << (3 * i + 2);
+    }
+  }
+  return m;
+}
+
 template <int kForm>
 __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
     scan_pair_kernel(const __grid_constant__ Params prm) {
@@ -1178,6 +1270,8 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
   {
     const uint32_t quarter = static_cast<uint32_t>(warp & 3);
     const uint32_t group = static_cast<uint32_t>(warp >> 2);
+    HitQueue* const queue = reinterpret_cast<HitQueue*>(smem_base + prm.queue_offset) + warp;
+    uint32_t queued = 0;
     const uint32_t lane_addr = (quarter * 32) << 16;
     auto chunk_any = [&](const uint32_t* raw, auto cols) -> uint32_t {
       constexpr int kCols = decltype(cols)::value;
@@ -1221,28 +1315,19 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
         x[i] = __float_as_uint(__fadd_rn(__uint_as_float(raw[i]), magic2_f));
       return (or_tree<kCols>(x) & 0x808080u) != 0;
     };
-    // the rare path: one lane's candidate masks of one chunk, bit i for triple i of the chunk
-    // (from v + MAGIC: bits 7 and 15, and field c's test on the whole value)
-    auto tri_masks = [&](const uint32_t* raw, auto cols, uint32_t (&m)[3]) {
-      constexpr int kCols = decltype(cols)::value;
-#pragma unroll
-      for (int i = 0; i < kCols; ++i) {
-        const uint32_t r = __float_as_uint(__fadd_rn(__uint_as_float(raw[i]), magic_f));
-        m[0] |= ((r >> 7) & 1u) << i;
-        m[1] |= ((r >> 15) & 1u) << i;
-        m[2] |= (r >= tc_bits ? 1u : 0u) << i;
-      }
-    };
     auto triple_tile = [&](uint32_t cols, uint64_t row, bool row_ok, uint64_t q_first,
                            uint32_t n_q, uint32_t (&raw0)[32], uint32_t (&raw1)[32],
                            float (&unused)[32], uint32_t ac) {
-      // chunk c (triples kChunkTriple[c] ..) of the group: its candidates re-checked exactly
-      // (all lanes take part)
-      auto report = [&](const uint32_t (&m)[3], uint32_t first_triple) {
+      // the rare path (all lanes take part)
+      auto report = [&](const uint32_t* raw, auto cols, uint32_t first_triple) {
+        constexpr int kCols = decltype(cols)::value;
 #pragma unroll
-        for (int f = 0; f < 3; ++f)
-          if (__any_sync(0xffffffffu, m[f] != 0))
-            emit_candidates_call(m[f], row, q_first + 3 * first_triple + f, n_q, &prm, lane, 3);
+        for (int c = 0; c < kCols; c += 8) {
+          const uint32_t m = triple_candidates(raw + c, row_ok, magic_f, tc_bits);
+          if (__any_sync(0xffffffffu, m != 0))
+            queued = push_candidates(m, row, 0, q_first + 3 * (first_triple + c), 1, n_q, queue,
+                                     queued, &prm, lane);
+        }
       };
       tmem_ld32_nowait(cols, raw0);
       tmem_ld32_nowait(cols + 32, raw1);
@@ -1251,15 +1336,10 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
       tmem_take(raw1, unused);
       const bool mine1 = row_ok & (tri_any(raw0, C32{}) | tri_any(raw1, C32{}));
       if (__any_sync(0xffffffffu, mine1)) {
-        // rare: report round 1's candidates now, while its columns are in registers (the
+        // rare: queue round 1's candidates now, while its columns are in registers (the
         // stage is handed back a little later)
-        uint32_t m0[3] = {}, m1[3] = {};
-        if (mine1) {
-          tri_masks(raw0, C32{}, m0);
-          tri_masks(raw1, C32{}, m1);
-        }
-        report(m0, 0);
-        report(m1, 32);
+        report(raw0, C32{}, 0);
+        report(raw1, C32{}, 32);
       }
       uint32_t raw2[16], raw3[8];
       tmem_ld32_nowait(cols + 64, raw0);
@@ -1275,16 +1355,10 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
       if (lane == 0) mbar_arrive(&sm.acc_empty[ac]);
       const bool mine2 =
           row_ok & (tri_any(raw0, C32{}) | tri_any(raw2, C16{}) | tri_any(raw3, C8{}));
-      uint32_t m2[3] = {}, m3[3] = {}, m4[3] = {};
-      if (mine2) {
-        tri_masks(raw0, C32{}, m2);
-        tri_masks(raw2, C16{}, m3);
-        tri_masks(raw3, C8{}, m4);
-      }
       if (__any_sync(0xffffffffu, mine2)) {
-        report(m2, 64);
-        report(m3, 96);
-        report(m4, 112);
+        report(raw0, C32{}, 64);
+        report(raw2, C16{}, 96);
+        report(raw3, C8{}, 112);
       }
     };
     uint32_t ga = 0;
@@ -1342,11 +1416,15 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.acc_empty[ac]);
-        // each chunk's candidates re-checked exactly (all lanes take part); the chunk starts
-        // at pair `pair` of the group
+        // each chunk's candidates (all lanes take part); the chunk starts at pair `pair` of the
+        // group
         auto report = [&](uint64_t m, uint32_t pair) {
-          if (__any_sync(0xffffffffu, m != 0))
-            emit_candidates_call(m, row, q_first + 2 * pair, n_queries, &prm, lane, 1);
+          const uint64_t q = q_first + 2 * pair;
+          if (!__any_sync(0xffffffffu, m != 0)) return;
+          queued = push_candidates(static_cast<uint32_t>(m), row, 0, q, 1, n_queries, queue,
+                                   queued, &prm, lane);
+          queued = push_candidates(static_cast<uint32_t>(m >> 32), row, 0, q + 32, 1, n_queries,
+                                   queue, queued, &prm, lane);
         };
         if (need1) {
           report(m0, 0);
@@ -1359,6 +1437,7 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
         }
       }
     }
+    flush_candidates(queue, queued, &prm, lane);
     if (!ok && lane == 0) raise_abort(sm, prm.dev_err);
     tc_fence_before();
     __syncwarp();
@@ -1393,12 +1472,11 @@ constexpr int kRowsMaxQueries = kTileRows;   // queries per launch (MMA M)
 // query q): the exact distance of each from popcounts, hits within the threshold written at
 // positions taken with one atomic per warp. Called by all 32 lanes; a lane without
 // candidates passes cand = 0.
-// (stride: bit j of cand stands for row row0 + stride * j; 1 unless given.)
 __device__ __forceinline__ void emit_rows(uint64_t cand, uint64_t row0, uint32_t q,
-                                          const Params& prm, int lane, uint32_t stride = 1) {
+                                          const Params& prm, int lane) {
   {
     // bits whose row is past the end
-    const uint64_t lim = row0 >= prm.n_rows ? 0 : (prm.n_rows - row0 + stride - 1) / stride;
+    const uint64_t lim = row0 >= prm.n_rows ? 0 : prm.n_rows - row0;
     if (lim < 64) cand &= (1ull << lim) - 1;
   }
   uint4 q0 = make_uint4(0, 0, 0, 0), q1 = q0;
@@ -1410,7 +1488,7 @@ __device__ __forceinline__ void emit_rows(uint64_t cand, uint64_t row0, uint32_t
   uint64_t hits = 0;
   for (uint64_t m = cand; m; m &= m - 1) {
     const int j = __ffsll(static_cast<long long>(m)) - 1;
-    const uint4* rp = reinterpret_cast<const uint4*>(prm.rows + (row0 + stride * j) * 32);
+    const uint4* rp = reinterpret_cast<const uint4*>(prm.rows + (row0 + j) * 32);
     if (popc256(__ldg(rp), __ldg(rp + 1), q0, q1) <= prm.threshold) hits |= 1ull << j;
   }
   const uint32_t mine = static_cast<uint32_t>(__popcll(hits));
@@ -1429,9 +1507,9 @@ __device__ __forceinline__ void emit_rows(uint64_t cand, uint64_t row0, uint32_t
   for (uint64_t m = hits; m; m &= m - 1, ++pos) {
     if (pos >= prm.capacity) break;
     const int j = __ffsll(static_cast<long long>(m)) - 1;
-    const uint4* rp = reinterpret_cast<const uint4*>(prm.rows + (row0 + stride * j) * 32);
+    const uint4* rp = reinterpret_cast<const uint4*>(prm.rows + (row0 + j) * 32);
     ypdq_hit h;
-    h.index = row0 + stride * j;
+    h.index = row0 + j;
     h.query = q + prm.query_base;
     h.distance = popc256(__ldg(rp), __ldg(rp + 1), q0, q1);
     prm.hits[pos] = h;
@@ -1747,12 +1825,6 @@ __device__ __forceinline__ void expand_prefix_fp4(const uint4 w0, uint8_t* chunk
   }
 }
 
-// emit_rows out of line (the rare path; keeps the epilogue's registers for its loads)
-__device__ __noinline__ void emit_rows_call(uint64_t cand, uint64_t row0, uint32_t q,
-                                            const Params* prm, int lane, uint32_t stride) {
-  emit_rows(cand, row0, q, *prm, lane, stride);
-}
-
 __global__ void __launch_bounds__(threads_of(false), 1)
     scan_rows3_kernel(const __grid_constant__ Params prm) {
   extern __shared__ uint8_t smem_raw[];
@@ -2002,6 +2074,8 @@ __global__ void __launch_bounds__(threads_of(false), 1)
     const uint32_t lane_addr = (quarter * 32) << 16;
     const uint32_t q = quarter * 32 + lane;
     const bool q_ok = q < n_queries;
+    HitQueue* const queue = reinterpret_cast<HitQueue*>(smem_base + prm.queue_offset) + warp;
+    uint32_t queued = 0;
     const bool active = quarter * 32 < n_queries;
     // field c's test: the column's bits (a float in [2^23, 2^24)) reach 2^23 + 65536 (126 - t)
     const uint32_t tc_bits =
@@ -2015,16 +2089,6 @@ __global__ void __launch_bounds__(threads_of(false), 1)
       for (int i = 0; i < kCols; ++i)
         x[i] = __float_as_uint(__fadd_rn(__uint_as_float(raw[i]), magic2));
       return (or_tree<kCols>(x) & 0x808080u) != 0;
-    };
-    auto tri_masks = [&](const uint32_t* raw, auto cols, uint32_t (&m)[3]) {
-      constexpr int kCols = decltype(cols)::value;
-#pragma unroll
-      for (int i = 0; i < kCols; ++i) {
-        const uint32_t r = __float_as_uint(__fadd_rn(__uint_as_float(raw[i]), magic));
-        m[0] |= ((r >> 7) & 1u) << i;
-        m[1] |= ((r >> 15) & 1u) << i;
-        m[2] |= (r >= tc_bits ? 1u : 0u) << i;
-      }
     };
     using C8 = std::integral_constant<int, 8>;
     using C16 = std::integral_constant<int, 16>;
@@ -2048,11 +2112,15 @@ __global__ void __launch_bounds__(threads_of(false), 1)
       const uint32_t cols = tmem_base + lane_addr + ac * kPairStageCols + kGroupCols * group;
       // database row of field f of the group's column i: row_g + 3 i + f
       const uint64_t row_g = tile * kRows3Rows + 3ull * kGroupCols * group;
-      auto report = [&](const uint32_t (&m)[3], uint32_t first) {
+      auto report = [&](const uint32_t* raw, auto n, uint32_t first) {
+        constexpr int kCols = decltype(n)::value;
 #pragma unroll
-        for (int f = 0; f < 3; ++f)
-          if (__any_sync(0xffffffffu, m[f] != 0))
-            emit_rows_call(m[f], row_g + 3 * first + f, q, &prm, lane, 3);
+        for (int c = 0; c < kCols; c += 8) {
+          const uint32_t m = triple_candidates(raw + c, q_ok, magic, tc_bits);
+          if (__any_sync(0xffffffffu, m != 0))
+            queued = push_candidates(m, row_g + 3 * (first + c), 1, q, 0, n_queries, queue, queued,
+                                     &prm, lane);
+        }
       };
       uint32_t raw0[32], raw1[32];
       float unused[32];
@@ -2063,13 +2131,8 @@ __global__ void __launch_bounds__(threads_of(false), 1)
       tmem_take(raw1, unused);
       const bool mine1 = q_ok & (tri_any(raw0, C32{}) | tri_any(raw1, C32{}));
       if (__any_sync(0xffffffffu, mine1)) {
-        uint32_t m0[3] = {}, m1[3] = {};
-        if (mine1) {
-          tri_masks(raw0, C32{}, m0);
-          tri_masks(raw1, C32{}, m1);
-        }
-        report(m0, 0);
-        report(m1, 32);
+        report(raw0, C32{}, 0);
+        report(raw1, C32{}, 32);
       }
       uint32_t raw2[16], raw3[8];
       tmem_ld32_nowait(cols + 64, raw0);
@@ -2083,20 +2146,17 @@ __global__ void __launch_bounds__(threads_of(false), 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.acc_empty[ac]);
-      const bool mine2 =
-          q_ok & (tri_any(raw0, C32{}) | tri_any(raw2, C16{}) | tri_any(raw3, C8{}));
-      uint32_t m2[3] = {}, m3[3] = {}, m4[3] = {};
-      if (mine2) {
-        tri_masks(raw0, C32{}, m2);
-        tri_masks(raw2, C16{}, m3);
-        tri_masks(raw3, C8{}, m4);
-      }
-      if (__any_sync(0xffffffffu, mine2)) {
-        report(m2, 64);
-        report(m3, 96);
-        report(m4, 112);
+      const bool any2 = q_ok & tri_any(raw0, C32{});
+      const bool any3 = q_ok & (tri_any(raw2, C16{}) | tri_any(raw3, C8{}));
+      if (__any_sync(0xffffffffu, any2 | any3)) {
+        if (__any_sync(0xffffffffu, any2)) report(raw0, C32{}, 64);
+        if (__any_sync(0xffffffffu, any3)) {
+          report(raw2, C16{}, 96);
+          report(raw3, C8{}, 112);
+        }
       }
     }
+    flush_candidates(queue, queued, &prm, lane);
     if (!ok && lane == 0) raise_abort(sm, prm.dev_err);
     tc_fence_before();
     __syncwarp();
@@ -2160,13 +2220,14 @@ cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
       p.n_queries <= 4u * static_cast<uint32_t>(tc::kRowsMaxQueries)) {
     const size_t b_end = tc::kFixedBytes +
                          static_cast<size_t>(tc::kRows3BChunks) * tc::kRows3ChunkBytes;
-    size_t stages = (tc::kSmemLimit - 1024 - b_end) / tc::kRows3PackBytes;
+    size_t stages = (tc::kSmemLimit - 1024 - b_end - tc::kQueueBytes) / tc::kRows3PackBytes;
     if (stages > static_cast<size_t>(tc::kMaxPackStages)) stages = tc::kMaxPackStages;
     if (stages < 2) return cudaErrorInvalidConfiguration;
     prm.n_tile = tc::kRowsMaxQueries;
     prm.pack_stages = static_cast<uint32_t>(stages);
     prm.pack_offset = static_cast<uint32_t>(b_end);
-    const size_t smem = b_end + stages * tc::kRows3PackBytes + 1024;
+    prm.queue_offset = static_cast<uint32_t>(b_end + stages * tc::kRows3PackBytes);
+    const size_t smem = prm.queue_offset + tc::kQueueBytes + 1024;
     const uint64_t rtiles = (p.n_rows + tc::kRows3Rows - 1) / tc::kRows3Rows;
     const unsigned g = static_cast<unsigned>(rtiles < static_cast<uint64_t>(num_sms) ? rtiles : num_sms);
     for (uint32_t q0 = 0; q0 < p.n_queries; q0 += tc::kRowsMaxQueries) {
@@ -2223,11 +2284,12 @@ cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
     prm.b_offset = static_cast<uint32_t>(tc::kFixedBytes +
                                          static_cast<size_t>(tc::kPairAStages) * tc::kChunkBytes);
     const size_t b_end = prm.b_offset + 2 * static_cast<size_t>(tc::kPairN) * 128;
-    size_t stages = (tc::kSmemLimit - 1024 - b_end) / tc::kPackBytes;
+    size_t stages = (tc::kSmemLimit - 1024 - b_end - tc::kQueueBytes) / tc::kPackBytes;
     if (stages > static_cast<size_t>(tc::kMaxPackStages)) stages = tc::kMaxPackStages;
     prm.pack_stages = static_cast<uint32_t>(stages);
     prm.pack_offset = static_cast<uint32_t>(b_end);
-    const size_t smem = b_end + stages * tc::kPackBytes + 1024;
+    prm.queue_offset = static_cast<uint32_t>(b_end + stages * tc::kPackBytes);
+    const size_t smem = prm.queue_offset + tc::kQueueBytes + 1024;
     const unsigned g = static_cast<unsigned>(grid);
     if (form == tc::kFormFp4Triples)
       tc::scan_pair_kernel<tc::kFormFp4Triples><<<g, tc::pair_threads(true), smem, s>>>(prm);
