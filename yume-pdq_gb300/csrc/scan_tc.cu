@@ -302,68 +302,105 @@ __device__ __forceinline__ void emit_candidates(uint64_t cand, uint64_t row, uin
 // a queue at a time, one candidate per lane. Re-checking them where they were found (row and
 // query loads, popcounts, an atomic: ~1.1 us for one candidate, while the tile's accumulator
 // stage and with it the SM's MMAs waited) cost a 10M-row scan with 10,000 hits 150 us where
-// one without hits took 81; with the queues and the decode by eight columns 111 and 78 (64
-// queries), 720 queries 421 -> 339, 8,192 queries 3,852 -> 3,283, 1,024 clustered queries on
-// 100M rows with 1.02 M hits 6,321 -> 5,492.
-constexpr uint32_t kQueueHits = 64;  // flushed past 32: one step of a push adds at most 32
+// one without hits took 81; with the queues and the decode by eight columns 115 and 79 (64
+// queries), 720 queries 421 -> 345, 8,192 queries 3,852 -> 3,261; 100M clustered rows: 64
+// queries with 64,000 hits 1,193 -> 725, 1,024 queries with 1.02 M hits 6,321 -> 5,120. (A
+// queue of 64 with an atomic per 32 took 859 and 5,492.)
+// A queue entry is row << 10 | query, the query counted from the pass' (launch's) first one
+// (at most 720 of them), so a queue is flushed at the end of a pass.
+constexpr uint32_t kQueueHits = 96;
 struct HitQueue {
-  uint64_t row[kQueueHits];
-  uint32_t query[kQueueHits];
+  uint64_t first_query;  // the pass' first query, and how many queries there are from it on
+  uint32_t n_queries;
+  uint64_t entry[kQueueHits];
 };
 constexpr size_t kQueueBytes = kEpilogueWarps * sizeof(HitQueue);
 
-// Re-check the first `count` candidates of the warp's queue exactly and report the hits, with
-// one atomic per 32. Called by all 32 lanes.
-__device__ __noinline__ void flush_candidates(const HitQueue* queue, uint32_t count,
-                                              const Params* prm, int lane) {
+// Re-check the `count` candidates of the warp's queue exactly, 32 at a time, and report the hits
+// with one atomic: they move to the queue's front meanwhile, with their distances in the top
+// nine bits (a row index stays far below 2^45). Called by all 32 lanes. (Rolled loops: the
+// registers come out of those that hold a tile's columns.)
+__device__ __noinline__ void flush_candidates(HitQueue* queue, uint32_t count, const Params* prm) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t n = 0;
   __syncwarp();
-  for (uint32_t at = 0; at < count; at += 32) {
-    const bool mine = at + lane < count;
-    const uint64_t row = queue->row[mine ? at + lane : at];
-    const uint32_t query = queue->query[mine ? at + lane : at];
-    const uint4* rp = reinterpret_cast<const uint4*>(prm->rows + row * 32);
-    const uint4* qp = reinterpret_cast<const uint4*>(prm->queries + static_cast<uint64_t>(query) * 32);
+#pragma unroll 1
+  for (uint32_t at = lane; at - lane < count; at += 32) {
+    // (a lane past the end takes its 32's first: entries before that may be hits already)
+    const uint64_t e = queue->entry[at < count ? at : at - lane];
+    const uint4* rp = reinterpret_cast<const uint4*>(prm->rows + (e >> 10) * 32);
+    const uint4* qp = reinterpret_cast<const uint4*>(
+        prm->queries + (queue->first_query + (e & 1023u)) * 32);
     const uint32_t d = popc256(__ldg(rp), __ldg(rp + 1), __ldg(qp), __ldg(qp + 1));
-    const bool hit = mine && d <= prm->threshold;
+    const bool hit = at < count && d <= prm->threshold;
     const uint32_t hits = __ballot_sync(0xffffffffu, hit);
-    if (hits == 0) continue;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(prm->count, static_cast<unsigned long long>(__popc(hits)));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    const uint64_t pos = base + __popc(hits & lanemask_lt());
-    if (hit && pos < prm->capacity) {
-      ypdq_hit h;
-      h.index = row;
-      h.query = query + prm->query_base;
-      h.distance = d;
-      prm->hits[pos] = h;
-    }
+    if (hit)
+      queue->entry[n + __popc(hits & lanemask_lt())] = static_cast<uint64_t>(d) << 55 | e;
+    n += __popc(hits);
+    __syncwarp();
+  }
+  if (n == 0) return;
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(prm->count, static_cast<unsigned long long>(n));
+  base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll 1
+  for (uint32_t at = lane; at < n && base + at < prm->capacity; at += 32) {
+    const uint64_t e = queue->entry[at];
+    ypdq_hit h;
+    h.index = (e >> 10) & ((1ull << 45) - 1);
+    h.query = static_cast<uint32_t>(queue->first_query + (e & 1023u)) + prm->query_base;
+    h.distance = static_cast<uint32_t>(e >> 55);
+    prm->hits[base + at] = h;
   }
   __syncwarp();
 }
 
-// Queue this lane's candidates: bit j of m is row `row + row_step * j` against query
-// `query + query_step * j` (those past the last row or query are dropped). Called by all 32
-// lanes; returns the queue's new count.
-__device__ __noinline__ uint32_t push_candidates(uint32_t m, uint64_t row, uint32_t row_step,
-                                                 uint64_t query, uint32_t query_step,
-                                                 uint32_t n_queries, HitQueue* queue,
-                                                 uint32_t count, const Params* prm, int lane) {
-  while (__any_sync(0xffffffffu, m != 0)) {
-    const int j = __ffs(static_cast<int>(m)) - 1;
-    const uint64_t r = row + static_cast<uint64_t>(row_step) * j;
-    const uint64_t q = query + static_cast<uint64_t>(query_step) * j;
-    const bool have = m != 0 && r < prm->n_rows && q < n_queries;
-    m &= m - 1;
-    const uint32_t all = __ballot_sync(0xffffffffu, have);
-    if (have) {
-      const uint32_t pos = count + __popc(all & lanemask_lt());
-      queue->row[pos] = r;
-      queue->query[pos] = static_cast<uint32_t>(q);
+// Queue this lane's candidates m: bit j is row `row + j` against the pass' query `query`
+// (kRows) or row `row` against its query `query + j`; bits past the last row or query are
+// dropped. Called by all 32 lanes; returns the queue's new count. (Few arguments: the calls'
+// registers come out of those that hold a tile's columns.)
+template <bool kRows>
+__device__ __noinline__ uint32_t push_candidates(uint32_t m, uint64_t row, uint32_t query,
+                                                 HitQueue* queue, uint32_t count,
+                                                 const Params* prm) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t end = kRows ? prm->n_rows : queue->n_queries, at = kRows ? row : query;
+  const uint64_t limit = at < end ? end - at : 0;
+  if (limit < 32) m &= (1u << limit) - 1u;
+  const uint64_t first = row << 10 | query;
+  constexpr uint64_t kStep = kRows ? 1u << 10 : 1u;
+  const uint32_t any = __ballot_sync(0xffffffffu, m != 0);
+  uint32_t before = __popc(any & lanemask_lt()), total = __popc(any);
+  if (__any_sync(0xffffffffu, (m & (m - 1)) != 0)) {
+    // lanes with several: prefix sums (in the usual case one lane has one)
+    uint32_t incl = __popc(m);
+#pragma unroll 1
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
     }
+    before = incl - __popc(m);
+    total = __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (count + total > kQueueHits) {
+    flush_candidates(queue, count, prm);
+    count = 0;
+  }
+  if (total <= kQueueHits) {
+    for (uint32_t pos = count + before; m; m &= m - 1)
+      queue->entry[pos++] = first + kStep * static_cast<uint32_t>(__ffs(static_cast<int>(m)) - 1);
+    return count + total;
+  }
+  // more than a queue's worth: a candidate of each lane at a time
+  while (__any_sync(0xffffffffu, m != 0)) {
+    const uint32_t all = __ballot_sync(0xffffffffu, m != 0);
+    if (m)
+      queue->entry[count + __popc(all & lanemask_lt())] =
+          first + kStep * static_cast<uint32_t>(__ffs(static_cast<int>(m)) - 1);
+    m &= m - 1;
     count += __popc(all);
     if (count > kQueueHits - 32) {
-      flush_candidates(queue, count, prm, lane);
+      flush_candidates(queue, count, prm);
       count = 0;
     }
   }
@@ -1315,8 +1352,9 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
         x[i] = __float_as_uint(__fadd_rn(__uint_as_float(raw[i]), magic2_f));
       return (or_tree<kCols>(x) & 0x808080u) != 0;
     };
-    auto triple_tile = [&](uint32_t cols, uint64_t row, bool row_ok, uint64_t q_first,
-                           uint32_t n_q, uint32_t (&raw0)[32], uint32_t (&raw1)[32],
+    // q_first: the group's first query in the pass
+    auto triple_tile = [&](uint32_t cols, uint64_t row, bool row_ok, uint32_t q_first,
+                           uint32_t (&raw0)[32], uint32_t (&raw1)[32],
                            float (&unused)[32], uint32_t ac) {
       // the rare path (all lanes take part)
       auto report = [&](const uint32_t* raw, auto cols, uint32_t first_triple) {
@@ -1325,8 +1363,8 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
         for (int c = 0; c < kCols; c += 8) {
           const uint32_t m = triple_candidates(raw + c, row_ok, magic_f, tc_bits);
           if (__any_sync(0xffffffffu, m != 0))
-            queued = push_candidates(m, row, 0, q_first + 3 * (first_triple + c), 1, n_q, queue,
-                                     queued, &prm, lane);
+            queued = push_candidates<false>(m, row, q_first + 3 * (first_triple + c), queue, queued,
+                                            &prm);
         }
       };
       tmem_ld32_nowait(cols, raw0);
@@ -1364,7 +1402,12 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
     uint32_t ga = 0;
     bool ok = true;
     for (uint32_t p = 0; p < n_passes && ok; ++p) {
-      const uint64_t pass_q = static_cast<uint64_t>(p) * kQueries;
+      if (lane == 0) {
+        const uint64_t pass_q = static_cast<uint64_t>(p) * kQueries;
+        queue->first_query = pass_q;
+        queue->n_queries = static_cast<uint32_t>(n_queries - pass_q);
+      }
+      __syncwarp();
       for (uint64_t k = 0; k < my_tiles; ++k, ++ga) {
         const uint64_t tile = blockIdx.x + k * gridDim.x;
         const uint32_t ac = ga % kAccStages;
@@ -1376,12 +1419,11 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
         const uint64_t row = tile * kTileRows + quarter * 32 + lane;
         const bool row_ok = row < prm.n_rows;
         const uint32_t cols = tmem_base + lane_addr + ac * kPairStageCols + kGroupCols * group;
-        const uint64_t q_first =
-            pass_q + (kTriples ? 3 : 2) * static_cast<uint64_t>(kGroupCols * group);
+        const uint32_t q_first = (kTriples ? 3 : 2) * kGroupCols * group;
         uint32_t raw0[32], raw1[32];
         float unused[32];
         if constexpr (kTriples) {
-          triple_tile(cols, row, row_ok, q_first, n_queries, raw0, raw1, unused, ac);
+          triple_tile(cols, row, row_ok, q_first, raw0, raw1, unused, ac);
           continue;
         }
         // round 1: pairs 0..63 of the group
@@ -1419,12 +1461,11 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
         // each chunk's candidates (all lanes take part); the chunk starts at pair `pair` of the
         // group
         auto report = [&](uint64_t m, uint32_t pair) {
-          const uint64_t q = q_first + 2 * pair;
           if (!__any_sync(0xffffffffu, m != 0)) return;
-          queued = push_candidates(static_cast<uint32_t>(m), row, 0, q, 1, n_queries, queue,
-                                   queued, &prm, lane);
-          queued = push_candidates(static_cast<uint32_t>(m >> 32), row, 0, q + 32, 1, n_queries,
-                                   queue, queued, &prm, lane);
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h)
+            queued = push_candidates<false>(static_cast<uint32_t>(m >> (32 * h)), row,
+                                            q_first + 2 * pair + 32 * h, queue, queued, &prm);
         };
         if (need1) {
           report(m0, 0);
@@ -1436,8 +1477,9 @@ __global__ void __launch_bounds__(pair_threads(kForm != 0), 1)
 
         }
       }
+      flush_candidates(queue, queued, &prm);
+      queued = 0;
     }
-    flush_candidates(queue, queued, &prm, lane);
     if (!ok && lane == 0) raise_abort(sm, prm.dev_err);
     tc_fence_before();
     __syncwarp();
@@ -1773,7 +1815,7 @@ __global__ void __launch_bounds__(threads_of(false), 1) scan_rows_kernel(const P
 }
 
 // ---------------------------------------------------------------------------------------
-// scan_rows3_kernel: narrow passes (<= 128 queries a launch; the launcher runs up to 512 as
+// scan_rows3_kernel: narrow passes (<= 128 queries a launch; the launcher runs up to 384 as
 // launches of 128) at t <= 36 with three database rows per f32 accumulator column and
 // block-scaled FP4 operands.
 //
@@ -2076,6 +2118,8 @@ __global__ void __launch_bounds__(threads_of(false), 1)
     const bool q_ok = q < n_queries;
     HitQueue* const queue = reinterpret_cast<HitQueue*>(smem_base + prm.queue_offset) + warp;
     uint32_t queued = 0;
+    if (lane == 0) queue->first_query = 0;
+    __syncwarp();
     const bool active = quarter * 32 < n_queries;
     // field c's test: the column's bits (a float in [2^23, 2^24)) reach 2^23 + 65536 (126 - t)
     const uint32_t tc_bits =
@@ -2118,8 +2162,7 @@ __global__ void __launch_bounds__(threads_of(false), 1)
         for (int c = 0; c < kCols; c += 8) {
           const uint32_t m = triple_candidates(raw + c, q_ok, magic, tc_bits);
           if (__any_sync(0xffffffffu, m != 0))
-            queued = push_candidates(m, row_g + 3 * (first + c), 1, q, 0, n_queries, queue, queued,
-                                     &prm, lane);
+            queued = push_candidates<true>(m, row_g + 3 * (first + c), q, queue, queued, &prm);
         }
       };
       uint32_t raw0[32], raw1[32];
@@ -2156,7 +2199,7 @@ __global__ void __launch_bounds__(threads_of(false), 1)
         }
       }
     }
-    flush_candidates(queue, queued, &prm, lane);
+    flush_candidates(queue, queued, &prm);
     if (!ok && lane == 0) raise_abort(sm, prm.dev_err);
     tc_fence_before();
     __syncwarp();
@@ -2182,6 +2225,51 @@ cudaError_t scan_tc_init() {
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+namespace tc {
+constexpr uint32_t kPassQueries = 3 * kPairFp4N;
+// Whether up to 719 queries cost less as launches of scan_rows3_kernel than as a pass of
+// scan_pair_kernel (`alone`: a launch of its own). In microseconds, with x million rows and no
+// hits: 8 + 7.0 x a launch of 128 queries, 27.2 x a pass however many queries it holds (144,
+// 176 or 208 columns instead of 240 took 260, 273 and 286 us on 10M rows: a tile is bound by
+// its accumulator stages' turnaround, not by N) and 1.4 for another pass or 10.5 for the first.
+// Measured, launches against a pass: 256 queries 18 / 13 us on 0.1M rows, 32 / 39 on 1M, 148 /
+// 276 on 10M; 384 queries 68 / 64 on 2M, 106 / 119 on 4M; 512 queries 292 / 282 on 10M. After
+// a full pass 304 queries on 10M rows 499 / 552 us in all, 82 / 66 on 1M.
+static bool rows3_pays(uint32_t queries, uint64_t n_rows, bool alone) {
+  const uint32_t launches = (queries + kRowsMaxQueries - 1) / kRowsMaxQueries;
+  const double x = 1e-6 * static_cast<double>(n_rows);
+  return launches * (8.0 + 7.0 * x) < (alone ? 10.5 : 1.4) + 27.2 * x;
+}
+}  // namespace tc
+
+bool scan_tc_runs_rows3(uint32_t n_queries, uint64_t n_rows) {
+  return n_queries < tc::kPassQueries && tc::rows3_pays(n_queries, n_rows, true);
+}
+
+// scan_pair_kernel over the first n_queries queries of prm, in one launch.
+static cudaError_t launch_pair_passes(tc::Params prm, uint32_t n_queries, int form, unsigned grid,
+                                      cudaStream_t s) {
+  prm.n_queries = n_queries;
+  prm.n_tile = static_cast<uint32_t>(tc::form_queries(form));
+  prm.a_stages = tc::kPairAStages;
+  // layout: [fixed Smem][A: 4 x 16 KB][B: 2 x 256 pairs x 128 B][packed ring][candidate queues],
+  // 1024-aligned
+  prm.b_offset = static_cast<uint32_t>(tc::kFixedBytes +
+                                       static_cast<size_t>(tc::kPairAStages) * tc::kChunkBytes);
+  const size_t b_end = prm.b_offset + 2 * static_cast<size_t>(tc::kPairN) * 128;
+  size_t stages = (tc::kSmemLimit - 1024 - b_end - tc::kQueueBytes) / tc::kPackBytes;
+  if (stages > static_cast<size_t>(tc::kMaxPackStages)) stages = tc::kMaxPackStages;
+  prm.pack_stages = static_cast<uint32_t>(stages);
+  prm.pack_offset = static_cast<uint32_t>(b_end);
+  prm.queue_offset = static_cast<uint32_t>(b_end + stages * tc::kPackBytes);
+  const size_t smem = prm.queue_offset + tc::kQueueBytes + 1024;
+  if (form == tc::kFormFp4Triples)
+    tc::scan_pair_kernel<tc::kFormFp4Triples><<<grid, tc::pair_threads(true), smem, s>>>(prm);
+  else
+    tc::scan_pair_kernel<tc::kFormFp8Pairs><<<grid, tc::pair_threads(false), smem, s>>>(prm);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
@@ -2211,13 +2299,19 @@ cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
   const bool half_k = p.threshold <= 36;
   const uint64_t tiles = (p.n_rows + tc::kTileRows - 1) / tc::kTileRows;
   const uint64_t grid = tiles < static_cast<uint64_t>(num_sms) ? tiles : num_sms;
-  // At t <= 36 with no pass width or FP8 pairs asked for, up to 512 queries: queries as A,
-  // three database rows per accumulator column (scan_rows3_kernel), one launch per 128
-  // queries. On 10M rows a launch takes 0.072-0.079 ms for 1 to 128 queries, so 2 to 4 of
-  // them beat one 256-query pass of scan_tc_kernel (0.23 ms) and one 720-query triple pass
-  // (0.327 ms); past 512 queries the triple passes cost less.
-  if (half_k && !p.n_tile && p.pair_n != static_cast<uint32_t>(tc::kPairN) &&
-      p.n_queries <= 4u * static_cast<uint32_t>(tc::kRowsMaxQueries)) {
+  // At t <= 36 with no pass width or FP8 pairs asked for: passes of 720 queries in triples
+  // (scan_pair_kernel), and the queries past the last full pass as launches of 128 with the
+  // queries as A (scan_rows3_kernel) or as one more pass, whichever takes less.
+  const uint32_t whole = p.n_queries / tc::kPassQueries * tc::kPassQueries;
+  const uint32_t rest = p.n_queries - whole;
+  if (half_k && !p.n_tile && p.pair_n != static_cast<uint32_t>(tc::kPairN) && rest > 0 &&
+      tc::rows3_pays(rest, p.n_rows, whole == 0)) {
+    if (whole) {
+      const cudaError_t e = launch_pair_passes(prm, whole, tc::kFormFp4Triples,
+                                               static_cast<unsigned>(grid), s);
+      if (e != cudaSuccess) return e;
+      prm.stall = 0;
+    }
     const size_t b_end = tc::kFixedBytes +
                          static_cast<size_t>(tc::kRows3BChunks) * tc::kRows3ChunkBytes;
     size_t stages = (tc::kSmemLimit - 1024 - b_end - tc::kQueueBytes) / tc::kRows3PackBytes;
@@ -2230,7 +2324,7 @@ cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
     const size_t smem = prm.queue_offset + tc::kQueueBytes + 1024;
     const uint64_t rtiles = (p.n_rows + tc::kRows3Rows - 1) / tc::kRows3Rows;
     const unsigned g = static_cast<unsigned>(rtiles < static_cast<uint64_t>(num_sms) ? rtiles : num_sms);
-    for (uint32_t q0 = 0; q0 < p.n_queries; q0 += tc::kRowsMaxQueries) {
+    for (uint32_t q0 = whole; q0 < p.n_queries; q0 += tc::kRowsMaxQueries) {
       tc::Params c = prm;
       c.queries = p.queries + static_cast<size_t>(q0) * 32;
       c.n_queries = p.n_queries - q0 < static_cast<uint32_t>(tc::kRowsMaxQueries)
@@ -2238,7 +2332,7 @@ cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
                         : static_cast<uint32_t>(tc::kRowsMaxQueries);
       c.query_base = p.query_base + q0;
       c.nq_off = q0;
-      c.stall = q0 == 0 ? prm.stall : 0;
+      c.stall = q0 == whole ? prm.stall : 0;
       tc::scan_rows3_kernel<<<g, tc::threads_of(false), smem, s>>>(c);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
@@ -2271,32 +2365,15 @@ cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
   if (p.pair_n && (!half_k || (p.pair_n != static_cast<uint32_t>(tc::kPairN) &&
                                 p.pair_n != kPairFp4N)))
     return cudaErrorInvalidValue;  // pairs need the 128-bit bound (t <= 36)
-  // at t <= 36 past 512 queries (or when asked for): several queries per accumulator column
+  // at t <= 36 without a pass width: several queries per accumulator column
   // (scan_pair_kernel), FP4 triples in passes of 720 or, with pair_n = 256, FP8 pairs in
-  // passes of 512. A triple pass costs less than a pair pass (0.327 against 0.36 ms on 10M
+  // passes of 512. A triple pass costs less than a pair pass (0.28 against 0.36 ms on 10M
   // rows) and covers more queries, so without a form asked for the triples run.
-  if (half_k && !p.n_tile && (p.pair_n || p.n_queries > static_cast<uint32_t>(tc::kMaxN))) {
-    const int form = p.pair_n == static_cast<uint32_t>(tc::kPairN) ? tc::kFormFp8Pairs
-                                                                   : tc::kFormFp4Triples;
-    prm.n_tile = static_cast<uint32_t>(tc::form_queries(form));
-    prm.a_stages = tc::kPairAStages;
-    // layout: [fixed Smem][A: 4 x 16 KB][B: 2 x 256 pairs x 128 B][packed ring], 1024-aligned
-    prm.b_offset = static_cast<uint32_t>(tc::kFixedBytes +
-                                         static_cast<size_t>(tc::kPairAStages) * tc::kChunkBytes);
-    const size_t b_end = prm.b_offset + 2 * static_cast<size_t>(tc::kPairN) * 128;
-    size_t stages = (tc::kSmemLimit - 1024 - b_end - tc::kQueueBytes) / tc::kPackBytes;
-    if (stages > static_cast<size_t>(tc::kMaxPackStages)) stages = tc::kMaxPackStages;
-    prm.pack_stages = static_cast<uint32_t>(stages);
-    prm.pack_offset = static_cast<uint32_t>(b_end);
-    prm.queue_offset = static_cast<uint32_t>(b_end + stages * tc::kPackBytes);
-    const size_t smem = prm.queue_offset + tc::kQueueBytes + 1024;
-    const unsigned g = static_cast<unsigned>(grid);
-    if (form == tc::kFormFp4Triples)
-      tc::scan_pair_kernel<tc::kFormFp4Triples><<<g, tc::pair_threads(true), smem, s>>>(prm);
-    else
-      tc::scan_pair_kernel<tc::kFormFp8Pairs><<<g, tc::pair_threads(false), smem, s>>>(prm);
-    return cudaGetLastError();
-  }
+  if (half_k && !p.n_tile)
+    return launch_pair_passes(prm, p.n_queries,
+                              p.pair_n == static_cast<uint32_t>(tc::kPairN) ? tc::kFormFp8Pairs
+                                                                            : tc::kFormFp4Triples,
+                              static_cast<unsigned>(grid), s);
   // passes of <= 128 queries: two MMA issuers and A in tensor memory (the pass is bound by
   // issuing and shared-memory traffic, not by the tensor core)
   const bool dual = prm.n_tile <= 128;
