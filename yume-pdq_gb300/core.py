@@ -1,6 +1,7 @@
 """Host-side objects over the C ABI: context, device buffers, batched hash and scan."""
 import ctypes
 import os
+import threading
 
 import numpy as np
 
@@ -21,9 +22,15 @@ class Context:
         check(self.lib.ypdq_device_info(h, ctypes.byref(sms), ctypes.byref(ctas)))
         self.num_sms = sms.value
         self.hash_ctas_per_sm = ctas.value
+        self._spare = []  # (pointer, bytes) of returned buffers, see borrow
+        self._spare_lock = threading.Lock()
 
     def close(self):
         if self.handle:
+            with self._spare_lock:
+                spare, self._spare = self._spare, []
+            for p, _ in spare:
+                self.lib.ypdq_free_device(self.handle, p)
             self.lib.ypdq_ctx_destroy(self.handle)
             self.handle = None
 
@@ -36,6 +43,29 @@ class Context:
     # -- memory
     def alloc(self, nbytes):
         return DeviceBuffer(self, nbytes)
+
+    # Buffers for the length of a call: cudaMalloc and cudaFree take ~20 us each, and the free
+    # waits for the device. At most SPARE_BUFFERS of up to SPARE_BYTES are kept, until close.
+    SPARE_BUFFERS, SPARE_BYTES = 8, 1 << 20
+
+    def borrow(self, nbytes):
+        """A device buffer of at least nbytes, to be given back with give_back once nothing on
+        the device uses it any more (or dropped, which frees it)."""
+        with self._spare_lock:
+            for i, (p, size) in enumerate(self._spare):
+                # a large buffer is not spent on a small need
+                if nbytes <= size and (size <= 1 << 16 or nbytes > 1 << 16):
+                    del self._spare[i]
+                    return DeviceBuffer(self, size, p)
+        return DeviceBuffer(self, max(int(nbytes), 1 << 16))
+
+    def give_back(self, buf):
+        if buf.nbytes <= self.SPARE_BYTES:
+            with self._spare_lock:
+                if self.handle and len(self._spare) < self.SPARE_BUFFERS:
+                    self._spare.append((buf.ptr, buf.nbytes))
+                    buf.ptr = None
+        buf.free()
 
     def to_device(self, array, stream=None):
         a = np.ascontiguousarray(array)
@@ -71,9 +101,12 @@ class Context:
 class DeviceBuffer:
     """Device memory from ypdq_malloc_device; freed with the object."""
 
-    def __init__(self, ctx, nbytes):
+    def __init__(self, ctx, nbytes, ptr=None):
         self.ctx = ctx
         self.nbytes = int(nbytes)
+        if ptr is not None:  # memory of this context that the object takes over
+            self.ptr = ptr
+            return
         p = ctypes.c_void_p()
         check(ctx.lib.ypdq_malloc_device(ctx.handle, max(self.nbytes, 1), ctypes.byref(p)))
         self.ptr = p
@@ -374,7 +407,7 @@ def screen_host(ctx, db, images, threshold=31, semantics="exact", dct=_lib.DCT_F
     imgs, kind = input_kind_of(images)
     n = imgs.shape[0]
     while True:
-        hits = np.zeros(max(capacity, 1), HIT_DTYPE)
+        hits = np.empty(max(capacity, 1), HIT_DTYPE)  # only what the call wrote is returned
         nh = ctypes.c_uint64()
         hashes = np.zeros((n, 8, 32), np.uint8) if want_hashes else None
         st = ctx.lib.ypdq_screen_host(ctx.handle, db.handle, ptr(imgs), n, kind, int(dct),

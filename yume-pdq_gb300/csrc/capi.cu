@@ -1,5 +1,6 @@
 // C ABI of libyumepdq_gb300: the batched device API (include/ypdq.h) and the drop-in
 // symbols of yume-pdq's C header (include/yume_pdq.h).
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -93,15 +94,14 @@ ypdq_status check_ctx(ypdq_ctx* ctx) {
   return YPDQ_OK;
 }
 
+// The error word is host memory that the kernels write through its device address, so after a
+// synchronisation reading it costs a load, not a blocking copy (~8 us).
 ypdq_status read_device_errors(ypdq_ctx* ctx) {
-  int err = 0;
-  CK(cudaMemcpy(&err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost), "read device errors");
-  if (err) {
-    CK(cudaMemset(ctx->d_err, 0, sizeof(int)), "clear device errors");
-    if (err & kDevErrTimeout)
-      return fail(YPDQ_ERR_TIMEOUT, "a kernel wait exceeded its time limit and gave up");
-    return fail(YPDQ_ERR_CUDA, "device error flags 0x%x", err);
-  }
+  if (*static_cast<volatile int*>(ctx->h_err) == 0) return YPDQ_OK;
+  const int err = __atomic_exchange_n(ctx->h_err, 0, __ATOMIC_ACQ_REL);
+  if (err & kDevErrTimeout)
+    return fail(YPDQ_ERR_TIMEOUT, "a kernel wait exceeded its time limit and gave up");
+  if (err) return fail(YPDQ_ERR_CUDA, "device error flags 0x%x", err);
   return YPDQ_OK;
 }
 
@@ -230,8 +230,11 @@ ypdq_status ypdq_ctx_create(int device, ypdq_ctx** out) {
     for (int d = 0; d < 3 && e == cudaSuccess; ++d)
       for (int sp = 0; sp < 2 && e == cudaSuccess; ++sp)
         e = hash_occupancy_variant(u, d, sp, &ctx->hash_ctas[u][d][sp]);
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaHostAlloc(&ctx->h_err, sizeof(int), cudaHostAllocMapped);
+  if (e == cudaSuccess) {
+    *ctx->h_err = 0;
+    e = cudaHostGetDevicePointer(&ctx->d_err, ctx->h_err, 0);
+  }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->jarosz_done, cudaEventDisableTiming);
@@ -247,12 +250,12 @@ ypdq_status ypdq_ctx_create(int device, ypdq_ctx** out) {
   for (int i = 0; i < ypdq_ctx::kMaxChunks && e == cudaSuccess; ++i)
     e = cudaEventCreateWithFlags(&ctx->chunk_copied[i], cudaEventDisableTiming);
   if (e != cudaSuccess) {
-    if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->h_err) cudaFreeHost(ctx->h_err);
     delete ctx;
     return cuda_fail(e, "ypdq_ctx_create");
   }
   if (ctx->hash_ctas_f32 < 1 || ctx->hash_ctas_u8 < 1) {
-    cudaFree(ctx->d_err);
+    cudaFreeHost(ctx->h_err);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return fail(YPDQ_ERR_UNSUPPORTED, "hash kernel does not fit on this device");
@@ -271,7 +274,7 @@ ypdq_status ypdq_ctx_destroy(ypdq_ctx* ctx) {
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   if (ctx->jarosz_done) cudaEventDestroy(ctx->jarosz_done);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
-  if (ctx->d_err) cudaFree(ctx->d_err);
+  if (ctx->h_err) cudaFreeHost(ctx->h_err);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   for (int i = 0; i < ypdq_ctx::kMaxChunks; ++i)
@@ -579,10 +582,14 @@ ypdq_status ypdq_screen_host(ypdq_ctx* ctx, ypdq_db* db, const void* h_images, i
     const int64_t i0 = bounds[c], i1 = bounds[c + 1];
     const uint8_t* src = static_cast<const uint8_t*>(h_images) + i0 * img_bytes;
     uint8_t* dst = static_cast<uint8_t*>(d_img) + i0 * img_bytes;
-    CK(cudaMemcpyAsync(dst, src, (i1 - i0) * img_bytes, cudaMemcpyHostToDevice, ctx->copy_stream),
-       "H2D images");
-    CK(cudaEventRecord(ctx->chunk_copied[c], ctx->copy_stream), "record copy");
-    CK(cudaStreamWaitEvent(s, ctx->chunk_copied[c], 0), "wait copy");
+    if (nch == 1) {  // nothing to overlap: no hand-over between streams
+      CK(cudaMemcpyAsync(dst, src, n * img_bytes, cudaMemcpyHostToDevice, s), "H2D images");
+    } else {
+      CK(cudaMemcpyAsync(dst, src, (i1 - i0) * img_bytes, cudaMemcpyHostToDevice, ctx->copy_stream),
+         "H2D images");
+      CK(cudaEventRecord(ctx->chunk_copied[c], ctx->copy_stream), "record copy");
+      CK(cudaStreamWaitEvent(s, ctx->chunk_copied[c], 0), "wait copy");
+    }
     HashLaunch hp{};
     hp.images = dst;
     hp.n = i1 - i0;
@@ -615,24 +622,40 @@ ypdq_status ypdq_screen_host(ypdq_ctx* ctx, ypdq_db* db, const void* h_images, i
     CK(launch_scan(sp, YPDQ_SCAN_AUTO, ctx->num_sms, s), "scan launch");
   }
   if (jarosz && n > 0) CK(cudaEventRecord(ctx->jarosz_done, s), "record jarosz scratch");
-  // results come back through the page-locked staging buffer: [count][error word][hits]
+  // results come back through the page-locked staging buffer: [count][hits][hashes][quality]
   uint8_t* stage = nullptr;
-  if ((st = host_stage(ctx, 64 + sizeof(ypdq_hit) * capacity, &stage))) return st;
+  const size_t hits_at = 64, hashes_at = hits_at + sizeof(ypdq_hit) * capacity;
+  const size_t quality_at = hashes_at + (h_hashes ? 256 * n : 0);
+  if ((st = host_stage(ctx, quality_at + (h_quality ? 32 * n : 0), &stage))) return st;
   CK(cudaMemcpyAsync(stage, d_cnt, sizeof(uint64_t), cudaMemcpyDeviceToHost, s), "D2H count");
-  CK(cudaMemcpyAsync(stage + 8, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H error word");
+  // the first hits come with the count: up to kHostSort are sorted here, without another round
+  // trip (~15 us with the sort's launch; sorting 128 hits on a core takes ~4)
+  constexpr uint64_t kHostSort = 128;
+  const uint64_t early = capacity < kHostSort ? capacity : kHostSort;
+  if (early > 0)
+    CK(cudaMemcpyAsync(stage + hits_at, d_hits, early * sizeof(ypdq_hit), cudaMemcpyDeviceToHost, s),
+       "D2H first hits");
+  if (h_hashes && n > 0) CK(cudaMemcpyAsync(stage + hashes_at, d_hash, 256 * n, cudaMemcpyDeviceToHost, s), "D2H hashes");
+  if (h_quality && n > 0) CK(cudaMemcpyAsync(stage + quality_at, d_q, 32 * n, cudaMemcpyDeviceToHost, s), "D2H quality");
   CK(cudaStreamSynchronize(s), "screen sync");
   uint64_t total = 0;
   memcpy(&total, stage, sizeof(total));
   const uint64_t m = total < capacity ? total : capacity;
-  CK(launch_sort_hits(static_cast<ypdq_hit*>(d_hits), m, ctx->pool, s), "sort launch");
-  if (m > 0) CK(cudaMemcpyAsync(stage + 64, d_hits, m * sizeof(ypdq_hit), cudaMemcpyDeviceToHost, s), "D2H hits");
-  if (h_hashes && n > 0) CK(cudaMemcpyAsync(h_hashes, d_hash, 256 * n, cudaMemcpyDeviceToHost, s), "D2H hashes");
-  if (h_quality && n > 0) CK(cudaMemcpyAsync(h_quality, d_q, 32 * n, cudaMemcpyDeviceToHost, s), "D2H quality");
-  CK(cudaStreamSynchronize(s), "screen sync");
-  if (m > 0) memcpy(h_hits, stage + 64, m * sizeof(ypdq_hit));
-  int dev_err = 0;
-  memcpy(&dev_err, stage + 8, sizeof(dev_err));
-  if (dev_err && (st = read_device_errors(ctx))) return st;
+  const bool all_here = m <= early;
+  if (all_here) {
+    ypdq_hit* const h = reinterpret_cast<ypdq_hit*>(stage + hits_at);
+    std::sort(h, h + m, [](const ypdq_hit& a, const ypdq_hit& b) {
+      return a.index != b.index ? a.index < b.index : a.query < b.query;
+    });
+  } else {
+    CK(launch_sort_hits(static_cast<ypdq_hit*>(d_hits), m, ctx->pool, s), "sort launch");
+    CK(cudaMemcpyAsync(stage + hits_at, d_hits, m * sizeof(ypdq_hit), cudaMemcpyDeviceToHost, s), "D2H hits");
+  }
+  if (h_hashes && n > 0) memcpy(h_hashes, stage + hashes_at, 256 * n);
+  if (h_quality && n > 0) memcpy(h_quality, stage + quality_at, 32 * n);
+  if (!all_here) CK(cudaStreamSynchronize(s), "screen sync");
+  if (m > 0) memcpy(h_hits, stage + hits_at, m * sizeof(ypdq_hit));
+  if ((st = read_device_errors(ctx))) return st;
   *n_hits = total;
   if (total > capacity) return fail(YPDQ_ERR_OVERFLOW, "%llu hits > capacity %llu",
                                     (unsigned long long)total, (unsigned long long)capacity);

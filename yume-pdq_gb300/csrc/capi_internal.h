@@ -15,7 +15,8 @@ struct ypdq_ctx {
   int hash_ctas_f32 = 1;
   int hash_ctas_u8 = 1;
   int hash_ctas[4][3][2] = {};  // [input kind][dct precision][separable compress]
-  int* d_err = nullptr;
+  int* h_err = nullptr;  // error word of the kernels: mapped host memory
+  int* d_err = nullptr;  // its device address
   cudaStream_t stream = nullptr;       // compute stream of the blocking _host calls
   cudaStream_t copy_stream = nullptr;  // host->device copies that overlap that compute
   static constexpr int kMaxChunks = 32;
@@ -23,7 +24,7 @@ struct ypdq_ctx {
   std::mutex mu;                  // guards the scratch buffers below
   void* scratch[8] = {};
   size_t scratch_bytes[8] = {};
-  // page-locked host staging of ypdq_screen_host's results (count, error word, hits), so
+  // page-locked host staging of ypdq_screen_host's results (count, hits, hashes, qualities), so
   // its device-to-host copies never take the driver's path for pageable memory
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;

@@ -1816,7 +1816,7 @@ __global__ void __launch_bounds__(threads_of(false), 1) scan_rows_kernel(const P
 
 // ---------------------------------------------------------------------------------------
 // scan_rows3_kernel: narrow passes (<= 128 queries a launch; the launcher runs up to 384 as
-// launches of 128) at t <= 36 with three database rows per f32 accumulator column and
+// launches of 128, with a device-side count up to 512) at t <= 36 with three database rows per f32 accumulator column and
 // block-scaled FP4 operands.
 //
 // The triple form of scan_pair_kernel with the operands swapped: the queries (126-bit
@@ -2244,10 +2244,6 @@ static bool rows3_pays(uint32_t queries, uint64_t n_rows, bool alone) {
 }
 }  // namespace tc
 
-bool scan_tc_runs_rows3(uint32_t n_queries, uint64_t n_rows) {
-  return n_queries < tc::kPassQueries && tc::rows3_pays(n_queries, n_rows, true);
-}
-
 // scan_pair_kernel over the first n_queries queries of prm, in one launch.
 static cudaError_t launch_pair_passes(tc::Params prm, uint32_t n_queries, int form, unsigned grid,
                                       cudaStream_t s) {
@@ -2304,8 +2300,11 @@ cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s) {
   // queries as A (scan_rows3_kernel) or as one more pass, whichever takes less.
   const uint32_t whole = p.n_queries / tc::kPassQueries * tc::kPassQueries;
   const uint32_t rest = p.n_queries - whole;
+  // (With a device-side count n_queries is only a bound, and a launch past the count ends at
+  // once where a pass takes its full time: up to 512 queries always run as launches.)
+  const bool counted = p.nq_dev && p.n_queries <= 4u * static_cast<uint32_t>(tc::kRowsMaxQueries);
   if (half_k && !p.n_tile && p.pair_n != static_cast<uint32_t>(tc::kPairN) && rest > 0 &&
-      tc::rows3_pays(rest, p.n_rows, whole == 0)) {
+      (counted || tc::rows3_pays(rest, p.n_rows, whole == 0))) {
     if (whole) {
       const cudaError_t e = launch_pair_passes(prm, whole, tc::kFormFp4Triples,
                                                static_cast<unsigned>(grid), s);

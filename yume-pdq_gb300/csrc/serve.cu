@@ -463,7 +463,7 @@ ypdq_status autotune(ypdq_server* S) {
     const uint32_t nq = 8 * b.images;
     if (nq <= 64) cand.push_back(Bucket{b.images, YPDQ_SCAN_SIMT, 0, 0, 0.0f, 0});
     // the launcher's choice: at t <= 36 queries as A with three database rows per column (FP4,
-    // one launch per 128 queries) for a few launches and FP4 triple passes of 720 past that;
+    // one launch per 128 queries) up to 512 queries and FP4 triple passes of 720 past that;
     // above t = 36 queries as A (FP8) up to 128 queries, then one query per column
     cand.push_back(Bucket{b.images, YPDQ_SCAN_TC, 0, 0, 0.0f, 0});
     const uint32_t nq64 = (nq + 63u) & ~63u;
@@ -759,8 +759,7 @@ ypdq_status ypdq_server_get_stats(ypdq_server* S, ypdq_server_stats* o, int rese
       } else if (b.pair_n == 256) {
         kern = 1, width = 512;
       } else if (low_t) {
-        const bool rows3 = scan_tc_runs_rows3(nq, S->db->n_rows);
-        kern = rows3 ? 4 : 3, width = rows3 ? 128 : 3 * kPairFp4N;
+        kern = nq <= 512 ? 4 : 3, width = nq <= 512 ? 128 : 3 * kPairFp4N;
       } else if (nq <= 128) {
         kern = 2, width = 128;
       } else {

@@ -325,8 +325,6 @@ cudaError_t scan_tc_init();
 uint64_t scan_wait_limit_ns();
 bool take_scan_stall();
 cudaError_t launch_scan_tc(const ScanLaunch& p, int num_sms, cudaStream_t s);
-// whether launch_scan_tc runs a scan at t <= 36 without a form asked for by scan_rows3_kernel alone
-bool scan_tc_runs_rows3(uint32_t n_queries, uint64_t n_rows);
 
 // stages.cu: the Kernel trait's per-stage methods on n items
 cudaError_t stages_init();

@@ -19,7 +19,8 @@ class CudaVectorDatabase(core.Database):
 
 
 class CudaMatcher:
-    """PDQMatcher over a CudaVectorDatabase with a fixed threshold."""
+    """PDQMatcher over a CudaVectorDatabase with a fixed threshold. Calls borrow their device
+    buffers from the context, so threads can share a matcher."""
 
     InputDimension = 32
     NoFalseNegative = True
@@ -33,41 +34,53 @@ class CudaMatcher:
         self.haystack = haystack
         self.threshold = int(threshold)
         self.algo = algo
-        self._cnt = ctx.alloc(8)
 
     @staticmethod
     def ident():
         return "CUDA sm_103a exact matcher"
 
-    def _queries(self, needles):
+    def _launch(self, work, q, d_hits, capacity):
+        """Scan needles q, whose copy lies 64 bytes into `work`, and read the count (its first
+        8 bytes), which waits for the scan."""
+        d_rows, n = self.haystack.device_rows()
+        core.scan_device(self.ctx, d_rows, n, work.at(64), q.shape[0], self.threshold, d_hits,
+                         capacity, work, self.algo)
+        return int(work.download((1,), np.uint64)[0])
+
+    def _needles(self, needles):
+        """Needles [q, 32] u8 and a borrowed buffer with them; the copy runs ahead of the scan
+        on the same stream."""
         q = np.ascontiguousarray(needles, np.uint8).reshape(-1, 32)
-        return q, (self.ctx.to_device(q) if q.shape[0] else self.ctx.alloc(32))
+        work = self.ctx.borrow(64 + q.nbytes)
+        if q.shape[0]:
+            _lib.check(self.ctx.lib.ypdq_memcpy(self.ctx.handle, work.at(64), _lib.ptr(q), q.nbytes,
+                                                _lib.H2D, None))
+        return q, work
 
     def scan(self, needles):
         """True if any haystack row is within the threshold of any needle."""
-        q, d_q = self._queries(needles)
-        d_rows, n = self.haystack.device_rows()
-        core.scan_device(self.ctx, d_rows, n, d_q, q.shape[0], self.threshold, None, 0,
-                         self._cnt, self.algo)
-        self.ctx.sync()
-        return int(self._cnt.download((1,), np.uint64)[0]) > 0
+        q, work = self._needles(needles)
+        total = self._launch(work, q, None, 0)
+        self.ctx.give_back(work)
+        return total > 0
 
     def find_all(self, needles, capacity=1 << 16):
         """Every hit (index, query, distance), sorted by (index, query)."""
-        q, d_q = self._queries(needles)
-        d_rows, n = self.haystack.device_rows()
+        q, work = self._needles(needles)
         while True:
-            d_hits = self.ctx.alloc(max(capacity, 1) * 16)
-            core.scan_device(self.ctx, d_rows, n, d_q, q.shape[0], self.threshold, d_hits,
-                             capacity, self._cnt, self.algo)
-            self.ctx.sync()
-            total = int(self._cnt.download((1,), np.uint64)[0])
+            d_hits = self.ctx.borrow(max(capacity, 1) * 16)
+            total = self._launch(work, q, d_hits, capacity)
             if total <= capacity:
                 break
+            self.ctx.give_back(d_hits)
             capacity = total
         if total > 1:
             core.sort_hits_device(self.ctx, d_hits, total)
-        return d_hits.download((total,), _lib.HIT_DTYPE) if total else np.zeros(0, _lib.HIT_DTYPE)
+        hits = (d_hits.download((total,), _lib.HIT_DTYPE) if total
+                else np.zeros(0, _lib.HIT_DTYPE))
+        self.ctx.give_back(d_hits)
+        self.ctx.give_back(work)
+        return hits
 
     def find(self, needles, f):
         """Call f(haystack_index, needle_index) for hits in (index, needle) order until it
