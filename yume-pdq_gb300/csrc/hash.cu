@@ -26,17 +26,21 @@
 //   warp 5     epilogue: quality, exact medians, bits and dihedrals of image k while the
 //              compute warps already work on image k+1 (double-buffered PDQF).
 //
-// f32 input is bound by HBM (1,024 images 168 us, 6.4 TB/s). The others are bound by issue
-// slots (64 % busy with the two compute warps per scheduler that 167 registers allow), so
+// f32 input is bound by HBM (1,024 images 164 us, 6.6 TB/s). The others are bound by issue
+// slots and latency (two compute warps per scheduler at 127-147 registers), so
 // what counts is instructions per compressed value, ~130 of which 27 are its serial sum:
 //   * a 4-row group finishes one value and starts the next from one carried sum, so nothing
 //     is read or converted twice and a stage of 2-4 groups costs one wait and one release;
 //   * byte conversion and product are one fma, products and DCT accumulators go in packed
 //     pairs (an f32x2 instruction takes two cycles of the FMA pipe but one issue slot);
 //   * RGB pixels become luma where they are read, without a staging of their own.
-// 4,096 u8 images: 552 -> 375 us (10.9 M images/s); 801 RGB8 images 262 -> 154 us; u8 with
-// the separable compress and the BF16x3 DCT, 1,024 images: 133 -> 83 us. A third CTA per SM
-// (96 registers, spilling) was slower: 434 us.
+//   * the epilogue, which shares the issue slots, selects three key bits per round and stops
+//     at a bin of one key, two slots side by side (one bit per round over all 32 for four
+//     slots: 375 us below; one slot after another: 1.3 us more for a single wave).
+// 4,096 u8 images: 552 -> 346 us (11.8 M images/s); 801 RGB8 images 262 -> 148 us; u8 with
+// the separable compress and the BF16x3 DCT, 1,024 images: 133 -> 73 us. A third CTA per SM
+// (96 registers, spilling) was slower: 434 us. So were compress and DCT in warps of their own:
+// 388 us, with no gain at f32.
 #include <cuda_bf16.h>
 
 #include <cstring>
@@ -116,7 +120,7 @@ struct HashSmem {
   alignas(128) unsigned char ring[kNumStages][kStageBytes];
   alignas(16) float dt[128][16];  // dt[i + 1][k] = D[k][i]; row 0 is zero
   float t[16][129];               // DCT stage 1 result T = D * B
-  alignas(16) float p[2][256];    // PDQF, double-buffered between compute and epilogue
+  float p[2][16][17];             // PDQF, double-buffered between compute and epilogue
   uint64_t full[kNumStages];
   uint64_t empty[kNumStages];
   uint64_t pfull[2];
@@ -280,36 +284,75 @@ __device__ __forceinline__ float key_f32(uint32_t k) {
   return __uint_as_float(u);
 }
 
-// Exact 128th-smallest (rank 127) of four 256-value sets held 8 per lane: MSB-first
-// radix selection on order-preserving keys, one warp reduction per bit and set.
-__device__ __forceinline__ void select_rank127_x4(const float (&v)[4][8], float (&out)[4]) {
-  uint32_t key[4][8];
+// The rank-127 values of kSets sets of 256 held 8 per lane: MSB-first radix selection on
+// order-preserving keys, three bits at a time: each lane counts its keys per digit in eight
+// 4-bit counters (at most 8 each), which are widened to 16 bits and summed over the warp by
+// four independent reductions. Once the digit's bin holds one key, that key is the answer
+// (after 4 or 5 of the 11 rounds on images); the loop ends when every set has its answer.
+template <int kSets>
+__device__ __forceinline__ void select_rank127(const float (&v)[kSets][8], float (&out)[kSets]) {
+  uint32_t key[kSets][8], prefix[kSets];
+  int rank[kSets], width[kSets];  // the rank within the digit's bin, the keys in it
 #pragma unroll
-  for (int s = 0; s < 4; ++s)
+  for (int s = 0; s < kSets; ++s) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) key[s][e] = f32_key(v[s][e]);
-  uint32_t prefix[4] = {0u, 0u, 0u, 0u};
-  int rank[4] = {127, 127, 127, 127};
-  uint32_t decided = 0u;
-#pragma unroll 4
-  for (int bit = 31; bit >= 0; --bit) {
-    const uint32_t b = 1u << bit;
-    const uint32_t m = decided | b;
+    prefix[s] = 0u;
+    rank[s] = 127;
+  }
+  int shift = 29;
+#pragma unroll 1
+  for (;;) {
+    uint32_t two[kSets][4];  // digits i and i + 4 in 16-bit halves
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      uint32_t c = 0;
+    for (int s = 0; s < kSets; ++s) {
+      uint32_t counts = 0u;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) c += ((key[s][e] & m) == prefix[s]) ? 1u : 0u;
-      const int tot = static_cast<int>(__reduce_add_sync(0xffffffffu, c));
-      if (rank[s] >= tot) {
-        rank[s] -= tot;
-        prefix[s] |= b;
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t k = (key[s][e] ^ prefix[s]) >> shift;  // above 7: another prefix
+        counts += k < 8u ? 1u << (4 * k) : 0u;
       }
+      // (in the last round, shift 0 with two bits left, digits 4-7 are keys of another prefix;
+      // the rank lies below them)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        two[s][i] = __reduce_add_sync(0xffffffffu, (counts >> (4 * i)) & 0x000F000Fu);
     }
-    decided = m;
+    bool single = true;
+#pragma unroll
+    for (int s = 0; s < kSets; ++s) {
+      int below = 0, upto = 256, digit = 0, cum = 0;  // keys below and up to the rank's digit
+#pragma unroll
+      for (int d = 0; d < 8; ++d) {
+        cum += static_cast<int>((d & 4) ? two[s][d & 3] >> 16 : two[s][d & 3] & 0xFFFFu);
+        if (cum <= rank[s]) {
+          below = cum;
+          digit = d + 1;
+        } else {
+          upto = min(upto, cum);
+        }
+      }
+      prefix[s] |= static_cast<uint32_t>(digit) << shift;
+      width[s] = upto - below;
+      rank[s] -= below;
+      single = single && width[s] == 1;
+    }
+    if (shift == 0) break;
+    if (single) {
+#pragma unroll
+      for (int s = 0; s < kSets; ++s) {
+        uint32_t found = 0u;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          found |= ((key[s][e] ^ prefix[s]) >> shift) == 0u ? key[s][e] : 0u;
+        prefix[s] = __reduce_or_sync(0xffffffffu, found);
+      }
+      break;
+    }
+    shift = shift > 3 ? shift - 3 : 0;
   }
 #pragma unroll
-  for (int s = 0; s < 4; ++s) out[s] = key_f32(prefix[s]);
+  for (int s = 0; s < kSets; ++s) out[s] = key_f32(prefix[s]);
 }
 
 // Slot s of the 8 outputs: value at (r, c) is sign * (s < 4 ? P[r][c] : P[c][r]).
@@ -317,36 +360,42 @@ __device__ __forceinline__ void select_rank127_x4(const float (&v)[4][8], float 
 __device__ __forceinline__ bool slot_rows(int s) { return s == 2 || s == 3 || s == 5 || s == 6; }
 __device__ __forceinline__ bool slot_cols(int s) { return s == 1 || s == 2 || s == 6 || s == 7; }
 
+// Slot s as signs and strides over P (pitch 17): value (r, c) is P[r row + c col] with its sign bit
+// flipped where bit r of `rows` and bit c of `cols` differ (see slot_rows).
+struct SlotView {
+  const float* P;
+  int row, col;
+  uint32_t rows, cols;
+  __device__ __forceinline__ SlotView(const float* P_, int s, uint32_t rm, uint32_t cm)
+      : P(P_), row(s < 4 ? 17 : 1), col(s < 4 ? 1 : 17), rows(slot_rows(s) ? rm : 0u),
+        cols(slot_cols(s) ? cm : 0u) {}
+  __device__ __forceinline__ float at(int r, int c) const {
+    return __uint_as_float(__float_as_uint(P[r * row + c * col]) ^
+                           (((rows >> r) ^ (cols >> c)) << 31));
+  }
+};
+
 // Sum of gradients of slot s, summed sequentially in the reference order.
-__device__ float slot_gradient(const float* P, int s, uint32_t rm, uint32_t cm) {
-  const bool tr = s >= 4, ur = slot_rows(s), uc = slot_cols(s);
-  auto val = [&](int r, int c) -> float {
-    float x = tr ? P[c * 16 + r] : P[r * 16 + c];
-    bool neg = (ur && ((rm >> r) & 1u)) != (uc && ((cm >> c) & 1u));
-    return neg ? -x : x;
-  };
+__device__ float slot_gradient(const SlotView& m) {
   float g = 0.0f;
   float prev[16];
 #pragma unroll
-  for (int c = 0; c < 16; ++c) prev[c] = val(0, c);
+  for (int c = 0; c < 16; ++c) prev[c] = m.at(0, c);
 #pragma unroll 1
   for (int r = 0; r < 15; ++r) {
-    float nxt[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) nxt[c] = val(r + 1, c);
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
-      g = __fadd_rn(g, fabsf(__fsub_rn(prev[c], nxt[c])));
-      prev[c] = nxt[c];
+      const float next = m.at(r + 1, c);
+      g = __fadd_rn(g, fabsf(__fsub_rn(prev[c], next)));
+      prev[c] = next;
     }
   }
 #pragma unroll 1
   for (int r = 0; r < 16; ++r) {
-    float row[16];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) row[c] = val(r, c);
+    for (int c = 0; c < 16; ++c) prev[c] = m.at(r, c);
 #pragma unroll
-    for (int c = 0; c < 15; ++c) g = __fadd_rn(g, fabsf(__fsub_rn(row[c], row[c + 1])));
+    for (int c = 0; c < 15; ++c) g = __fadd_rn(g, fabsf(__fsub_rn(prev[c], prev[c + 1])));
   }
   return g;
 }
@@ -359,83 +408,54 @@ struct EpilogueOut {
   int pdqf_slots;
 };
 
-// One warp turns a PDQF held in shared memory into the 8 slot hashes, thresholds and
-// qualities. With thr0_given the slot-0 threshold is taken from the caller.
-__device__ void epilogue_warp(const float* P, bool thr0_given, float thr0_in, uint32_t rm,
-                              uint32_t cm, int lane, const EpilogueOut& o) {
-  // lane owns flat elements k = 8*lane + e, i.e. row i = lane/2, columns j0 .. j0+7
+// Medians, bits and outputs of slots s .. s + kSets - 1 and the four after each (s < 4; slot
+// s + 4 is slot s's transpose with the other axis' signs, at slot s's threshold) by one warp.
+// With thr_given the threshold of slot s is the caller's.
+template <int kSets>
+__device__ __forceinline__ void slot_pairs(const float* P, int s, uint32_t rm, uint32_t cm,
+                                           int lane, const EpilogueOut& o, bool thr_given,
+                                           float thr_in) {
   const int i = lane >> 1, j0 = (lane & 1) << 3;
-  const bool rneg = (rm >> i) & 1u;
-  float x[8], xt[8];
+  float v[kSets][8], thr[kSets];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    x[e] = P[i * 16 + j0 + e];
-    xt[e] = P[(j0 + e) * 16 + i];
+  for (int x = 0; x < kSets; ++x) {
+    const SlotView m(P, s + x, rm, cm);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[x][e] = m.at(i, j0 + e);
   }
-  float v[8][8];
+  select_rank127(v, thr);
+  if (thr_given) thr[0] = thr_in;
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const bool cneg = (cm >> (j0 + e)) & 1u;
-    const float cx = cneg ? -x[e] : x[e];
-    const float cxt = cneg ? -xt[e] : xt[e];
-    v[0][e] = x[e];
-    v[1][e] = cx;
-    v[2][e] = rneg ? -cx : cx;
-    v[3][e] = rneg ? -x[e] : x[e];
-    v[4][e] = xt[e];
-    v[5][e] = rneg ? -xt[e] : xt[e];
-    v[6][e] = rneg ? -cxt : cxt;
-    v[7][e] = cxt;
-  }
-  float med[4];
-  {
-    float sel[4][8];
+  for (int h = 0; h < 2 * kSets; ++h) {
+    const int x = h % kSets, slot = s + x + 4 * (h / kSets);
+    if (h >= kSets) {
+      const SlotView m(P, slot, rm, cm);
 #pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) sel[s][e] = v[s][e];
-    select_rank127_x4(sel, med);
-  }
-  float thr[8];
-  thr[0] = thr0_given ? thr0_in : med[0];
-  thr[1] = med[1];
-  thr[2] = med[2];
-  thr[3] = med[3];
-  thr[4] = thr[0];
-  thr[5] = thr[1];
-  thr[6] = thr[2];
-  thr[7] = thr[3];
-  if (o.hashes) {
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      uint32_t byte = 0;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) byte |= (v[s][e] > thr[s] ? 1u : 0u) << e;
-      o.hashes[s * 32 + 31 - lane] = static_cast<uint8_t>(byte);
+      for (int e = 0; e < 8; ++e) v[x][e] = m.at(i, j0 + e);
     }
-  }
-  if (o.pdqf) {
-    const int slots = o.pdqf_slots == 8 ? 8 : 1;
+    uint32_t byte = 0;
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      if (s < slots) {
-        float4* dst = reinterpret_cast<float4*>(o.pdqf + s * 256 + lane * 8);
-        dst[0] = make_float4(v[s][0], v[s][1], v[s][2], v[s][3]);
-        dst[1] = make_float4(v[s][4], v[s][5], v[s][6], v[s][7]);
-      }
+    for (int e = 0; e < 8; ++e) byte |= (v[x][e] > thr[x] ? 1u : 0u) << e;
+    if (o.hashes) o.hashes[slot * 32 + 31 - lane] = static_cast<uint8_t>(byte);
+    if (o.pdqf && (slot == 0 || o.pdqf_slots == 8)) {
+      float4* dst = reinterpret_cast<float4*>(o.pdqf + slot * 256 + lane * 8);
+      dst[0] = make_float4(v[x][0], v[x][1], v[x][2], v[x][3]);
+      dst[1] = make_float4(v[x][4], v[x][5], v[x][6], v[x][7]);
     }
+    if (o.thresholds && lane == 0) o.thresholds[slot] = thr[x];
   }
-  if (lane < 8) {
-    float t = thr[0];
-#pragma unroll
-    for (int s = 1; s < 8; ++s)
-      if (lane == s) t = thr[s];
-    if (o.thresholds) o.thresholds[lane] = t;
-    if (o.quality) {
-      const float g = slot_gradient(P, lane, rm, cm);
-      o.quality[lane] = fminf(__fdiv_rn(g, 180.0f), 1.0f);
-    }
-  }
+}
+
+// One warp turns a PDQF held in shared memory (16 rows at a pitch of 17) into the 8 slot hashes,
+// thresholds and qualities. With thr0_given the slot-0 threshold is taken from the caller.
+__device__ __forceinline__ void epilogue_warp(const float* P, bool thr0_given, float thr0_in,
+                                              uint32_t rm, uint32_t cm, int lane,
+                                              const EpilogueOut& o) {
+#pragma unroll 1
+  for (int s = 0; s < 4; s += 2)
+    slot_pairs<2>(P, s, rm, cm, lane, o, s == 0 && thr0_given, thr0_in);
+  if (o.quality && lane < 8)
+    o.quality[lane] = fminf(__fdiv_rn(slot_gradient(SlotView(P, lane, rm, cm)), 180.0f), 1.0f);
 }
 
 // ------------------------------------------------------------------- kernel
@@ -638,7 +658,7 @@ __global__ void __launch_bounds__(hash_threads<kDct>(), 2)
       o.thresholds = prm.thresholds ? prm.thresholds + n * 8 : nullptr;
       o.pdqf_slots = prm.pdqf_slots;
       o.pdqf = prm.pdqf ? prm.pdqf + n * (prm.pdqf_slots == 8 ? 8 : 1) * 256 : nullptr;
-      epilogue_warp(sm.p[pb], false, 0.0f, prm.row_mask, prm.col_mask, lane, o);
+      epilogue_warp(sm.p[pb][0], false, 0.0f, prm.row_mask, prm.col_mask, lane, o);
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.pempty[pb]);
     }
@@ -847,7 +867,8 @@ __global__ void __launch_bounds__(hash_threads<kDct>(), 2)
       const float2 p = add2_rn(add2_rn(add2_rn(sum[0], sum[1]), sum[2]), sum[3]);
       const int pb = it & 1;
       if (!mbar_wait(&sm.pempty[pb], ((it >> 1) & 1u) ^ 1u, abort_flag)) goto fail;
-      *reinterpret_cast<float2*>(&sm.p[pb][k * 16 + c0]) = p;
+      sm.p[pb][k][c0] = p.x;
+      sm.p[pb][k][c0 + 1] = p.y;
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.pfull[pb]);
     }
@@ -1004,69 +1025,6 @@ __device__ __forceinline__ void split_dct_stage(SplitSmem& sm, int stage, int ra
   }
 }
 
-// The rank-127 value of 256 held 8 per lane: MSB-first radix selection like
-// select_rank127_x4's, three bits at a time: each lane counts its keys per digit in eight
-// 4-bit counters (at most 8 each), which are widened to 16 bits and summed over the warp by
-// four independent reductions. Once the digit's bin holds one key, that key is the answer
-// (after 4 or 5 of the 11 rounds on images).
-__device__ __forceinline__ float select_rank127(const float (&v)[8]) {
-  uint32_t key[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) key[e] = f32_key(v[e]);
-  uint32_t prefix = 0u;
-  int rank = 127;
-#pragma unroll 1
-  for (int shift = 29;; shift = shift > 3 ? shift - 3 : 0) {
-    uint32_t counts = 0u;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const uint32_t k = (key[e] ^ prefix) >> shift;  // above 7: another prefix
-      counts += k < 8u ? 1u << (4 * k) : 0u;
-    }
-    // (in the last round, shift 0 with two bits left, digits 4-7 are keys of another prefix;
-    // the rank lies below them)
-    uint32_t two[4];  // digits i and i + 4 in 16-bit halves
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      two[i] = __reduce_add_sync(0xffffffffu, (counts >> (4 * i)) & 0x000F000Fu);
-    int below = 0, upto = 256, digit = 0, cum = 0;  // keys below and up to the rank's digit
-#pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      cum += static_cast<int>((d & 4) ? two[d & 3] >> 16 : two[d & 3] & 0xFFFFu);
-      if (cum <= rank) {
-        below = cum;
-        digit = d + 1;
-      } else {
-        upto = min(upto, cum);
-      }
-    }
-    prefix |= static_cast<uint32_t>(digit) << shift;
-    if (shift == 0) return key_f32(prefix);
-    if (upto - below == 1) {
-      uint32_t found = 0u;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) found |= ((key[e] ^ prefix) >> shift) == 0u ? key[e] : 0u;
-      return key_f32(__reduce_or_sync(0xffffffffu, found));
-    }
-    rank -= below;
-  }
-}
-
-// Slot s as signs and strides over P (pitch 17): value (r, c) is P[r row + c col] with its sign bit
-// flipped where bit r of `rows` and bit c of `cols` differ (see slot_rows).
-struct SlotView {
-  const float* P;
-  int row, col;
-  uint32_t rows, cols;
-  __device__ __forceinline__ SlotView(const float* P_, int s, uint32_t rm, uint32_t cm)
-      : P(P_), row(s < 4 ? 17 : 1), col(s < 4 ? 1 : 17), rows(slot_rows(s) ? rm : 0u),
-        cols(slot_cols(s) ? cm : 0u) {}
-  __device__ __forceinline__ float at(int r, int c) const {
-    return __uint_as_float(__float_as_uint(P[r * row + c * col]) ^
-                           (((rows >> r) ^ (cols >> c)) << 31));
-  }
-};
-
 // Quality of slot s by one warp: its 480 absolute differences in parallel into `g` in the
 // reference's order (240 down the columns, row by row, then 240 along the rows), then the
 // sequential sum in lane 0 (480 dependent additions, the loads 16 values ahead of them).
@@ -1110,35 +1068,6 @@ __device__ __forceinline__ void split_quality(const float* P, int s, uint32_t rm
       sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, b[q].x), b[q].y), b[q].z), b[q].w);
   }
   quality[s] = fminf(__fdiv_rn(sum, 180.0f), 1.0f);
-}
-
-// Median, bits and outputs of slots s and s + 4 (s < 4; slot s + 4 is slot s's transpose
-// with the other axis' signs, at slot s's threshold) by one warp.
-__device__ __forceinline__ void split_slots(const float* P, int s, uint32_t rm, uint32_t cm,
-                                            int lane, const EpilogueOut& o) {
-  const int i = lane >> 1, j0 = (lane & 1) << 3;
-  float v[2][8];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const SlotView m(P, s + 4 * h, rm, cm);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[h][e] = m.at(i, j0 + e);
-  }
-  const float thr = select_rank127(v[0]);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int slot = s + 4 * h;
-    uint32_t byte = 0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) byte |= (v[h][e] > thr ? 1u : 0u) << e;
-    if (o.hashes) o.hashes[slot * 32 + 31 - lane] = static_cast<uint8_t>(byte);
-    if (o.pdqf && (slot == 0 || o.pdqf_slots == 8)) {
-      float4* dst = reinterpret_cast<float4*>(o.pdqf + slot * 256 + lane * 8);
-      dst[0] = make_float4(v[h][0], v[h][1], v[h][2], v[h][3]);
-      dst[1] = make_float4(v[h][4], v[h][5], v[h][6], v[h][7]);
-    }
-    if (o.thresholds && lane == 0) o.thresholds[slot] = thr;
-  }
 }
 
 template <typename Tin>
@@ -1244,7 +1173,7 @@ __global__ void __cluster_dims__(kSplitCtas, 1, 1) __launch_bounds__(kSplitThrea
       o.thresholds = prm.thresholds ? prm.thresholds + n * 8 : nullptr;
       o.pdqf_slots = prm.pdqf_slots;
       o.pdqf = prm.pdqf ? prm.pdqf + n * (prm.pdqf_slots == 8 ? 8 : 1) * 256 : nullptr;
-      split_slots(sm.p[0], warp - 8, prm.row_mask, prm.col_mask, lane, o);
+      slot_pairs<1>(sm.p[0], warp - 8, prm.row_mask, prm.col_mask, lane, o, false, 0.0f);
     }
   }
   cluster_wait();
@@ -1252,14 +1181,20 @@ __global__ void __cluster_dims__(kSplitCtas, 1, 1) __launch_bounds__(kSplitThrea
 
 // Dihedrals of given PDQF matrices: one warp per matrix.
 __global__ void __launch_bounds__(128) dihedral_kernel(const DihedralLaunch prm) {
-  __shared__ __align__(16) float P[4][256];
+  __shared__ float P[4][16 * 17];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n = static_cast<int64_t>(blockIdx.x) * 4 + w;
   if (n >= prm.n) return;
   const float4* src = reinterpret_cast<const float4*>(prm.pdqf + n * 256);
-  float4* dst = reinterpret_cast<float4*>(P[w]);
-  dst[lane] = src[lane];
-  dst[lane + 32] = src[lane + 32];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float4 x = src[lane + 32 * h];
+    float* dst = &P[w][17 * ((lane + 32 * h) >> 2) + 4 * (lane & 3)];
+    dst[0] = x.x;
+    dst[1] = x.y;
+    dst[2] = x.z;
+    dst[3] = x.w;
+  }
   __syncwarp();
   EpilogueOut o;
   o.hashes = prm.hashes ? prm.hashes + n * 256 : nullptr;
