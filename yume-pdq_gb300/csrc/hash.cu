@@ -27,20 +27,24 @@
 //              compute warps already work on image k+1 (double-buffered PDQF).
 //
 // f32 input is bound by HBM (1,024 images 164 us, 6.6 TB/s). The others are bound by issue
-// slots and latency (two compute warps per scheduler at 127-147 registers), so
-// what counts is instructions per compressed value, ~130 of which 27 are its serial sum:
+// slots and latency (two compute warps per scheduler at 152 registers), so what counts is
+// instructions per compressed value, ~115, and how long its serial sum of 27 terms takes:
 //   * a 4-row group finishes one value and starts the next from one carried sum, so nothing
 //     is read or converted twice and a stage of 2-4 groups costs one wait and one release;
-//   * byte conversion and product are one fma, products and DCT accumulators go in packed
-//     pairs (an f32x2 instruction takes two cycles of the FMA pipe but one issue slot);
-//   * RGB pixels become luma where they are read, without a staging of their own.
+//   * byte input: two groups' sums go side by side in packed pairs (an f32x2 instruction takes
+//     two cycles of the FMA pipe but one issue slot): two values per 27 dependent adds (one
+//     value each: 346 us below, RGB8 148). f32 rows come as 16-byte loads whose pairs would
+//     have to be moved together, so f32 keeps the scalar sums;
+//   * byte conversion and product are one fma, and the DCT's accumulators are pairs as well;
+//   * RGB pixels become luma where they are read, without a staging of their own;
 //   * the epilogue, which shares the issue slots, selects three key bits per round and stops
 //     at a bin of one key, two slots side by side (one bit per round over all 32 for four
-//     slots: 375 us below; one slot after another: 1.3 us more for a single wave).
-// 4,096 u8 images: 552 -> 346 us (11.8 M images/s); 801 RGB8 images 262 -> 148 us; u8 with
-// the separable compress and the BF16x3 DCT, 1,024 images: 133 -> 73 us. A third CTA per SM
-// (96 registers, spilling) was slower: 434 us. So were compress and DCT in warps of their own:
-// 388 us, with no gain at f32.
+//     slots: 375 us before the pairs; one slot after another: 1.3 us more for a single wave).
+// 4,096 u8 images: 552 -> 324 us (12.6 M images/s); 801 RGB8 images 262 -> 136 us; u8 with
+// the separable compress and the BF16x3 DCT, 1,024 images: 133 -> 72 us. No gain, measured: a
+// third CTA per SM (128 registers, copies and epilogue in one warp: 342 us against 346, single
+// waves 4 us longer), compress and DCT in warps of their own (388 against 375 us, none at
+// f32), a pair's DCT steps put beside the next pair's sums (the same times).
 #include <cuda_bf16.h>
 
 #include <cstring>
@@ -240,6 +244,97 @@ __device__ __forceinline__ float compress_group(const Tin* rows, int j, bool las
   return done;
 }
 
+// The same five columns of two rows, paired row by row.
+struct RowX2 {
+  float2 v[5];
+};
+__device__ __forceinline__ RowX2 load_rows(const uint8_t* p, const uint8_t* q, int j) {
+  const uint32_t* r = reinterpret_cast<const uint32_t*>(p);
+  const uint32_t* s = reinterpret_cast<const uint32_t*>(q);
+  const uint32_t a = r[j], b = r[j + 1], c = s[j], d = s[j + 1];
+  return {make_float2(byte_biased<2>(a), byte_biased<2>(c)),
+          make_float2(byte_biased<3>(a), byte_biased<3>(c)),
+          make_float2(byte_biased<0>(b), byte_biased<0>(d)),
+          make_float2(byte_biased<1>(b), byte_biased<1>(d)),
+          make_float2(byte_biased<2>(b), byte_biased<2>(d))};
+}
+template <int kR, int kG, int kB>  // bytes of the two words' channels
+__device__ __forceinline__ float2 luma_rows(uint32_t r, uint32_t g, uint32_t b, uint32_t r1,
+                                            uint32_t g1, uint32_t b1) {
+  return luma2_bt601(make_float2(byte_biased<kR>(r), byte_biased<kR>(r1)),
+                     make_float2(byte_biased<kG>(g), byte_biased<kG>(g1)),
+                     make_float2(byte_biased<kB>(b), byte_biased<kB>(b1)));
+}
+__device__ __forceinline__ RowX2 load_rows(const rgb8_t* p, const rgb8_t* q, int j) {
+  // pixels 0-3 in three words: r g b r | g b r g | b r g b
+  const uint32_t* r = reinterpret_cast<const uint32_t*>(p) + 3 * j;
+  const uint32_t* s = reinterpret_cast<const uint32_t*>(q) + 3 * j;
+  return {luma_rows<2, 3, 0>(r[1], r[1], r[2], s[1], s[1], s[2]),
+          luma_rows<1, 2, 3>(r[2], r[2], r[2], s[2], s[2], s[2]),
+          luma_rows<0, 1, 2>(r[3], r[3], r[3], s[3], s[3], s[3]),
+          luma_rows<3, 0, 1>(r[3], r[4], r[4], s[3], s[4], s[4]),
+          luma_rows<2, 3, 0>(r[4], r[4], r[5], s[4], s[4], s[5])};
+}
+__device__ __forceinline__ RowX2 load_rows(const rgba8_t* p, const rgba8_t* q, int j) {
+  const uint4* r = reinterpret_cast<const uint4*>(p);
+  const uint4* s = reinterpret_cast<const uint4*>(q);
+  const uint4 a = r[j], b = r[j + 1], c = s[j], d = s[j + 1];
+  return {luma_rgba(a.z, c.z), luma_rgba(a.w, c.w), luma_rgba(b.x, d.x), luma_rgba(b.y, d.y),
+          luma_rgba(b.z, d.z)};
+}
+// RN(w x) of both rows. Packed adds take these products, so the multiply must be one that is
+// not contracted.
+template <typename T>
+__device__ __forceinline__ float2 weighted_both(float w, float2 x, float nz) {
+  if constexpr (sizeof(T) == 1)
+    return fma2_rn(make_float2(w, w), x, make_float2(-kByteBias * w, -kByteBias * w));
+  else
+    return mul2_rn(make_float2(w, w), x, nz);
+}
+template <typename T>
+__device__ __forceinline__ RowX2 weighted_rows(float w1, float w2, float w3, const RowX2& x,
+                                               float nz) {
+  return {weighted_both<T>(w1, x.v[0], nz), weighted_both<T>(w2, x.v[1], nz),
+          weighted_both<T>(w3, x.v[2], nz), weighted_both<T>(w2, x.v[3], nz),
+          weighted_both<T>(w1, x.v[4], nz)};
+}
+__device__ __forceinline__ float2 add_rows(float2 s, const RowX2& p) {
+#pragma unroll
+  for (int k = 0; k < 5; ++k) s = add2_rn(s, p.v[k]);
+  return s;
+}
+
+// Groups g and g + 1 (8 rows): finishes values g - 1 and g and starts value g + 1. The two
+// groups' sums go side by side in packed pairs (half the issue slots of the serial sums, and
+// twice the work between two steps of one); the finishing pair continues the sum carried in
+// and the one just started by group g. The last pair starts a value that does not exist from
+// whatever its two missing rows' place holds; nothing reads it.
+template <typename Tin>
+__device__ __forceinline__ float2 compress_pair(const Tin* rows, int j, bool last, float nz,
+                                                TapSum& c) {
+  if constexpr (std::is_same<Tin, float>::value) {
+    const float a = compress_group(rows, j, false, c);
+    return make_float2(a, compress_group(rows + 4 * 512, j, last, c));
+  } else {
+    using T = typename std::conditional<is_rgb<Tin>(), float, Tin>::type;
+    const Tin* second = rows + 4 * 512;
+    const RowX2 x = load_rows(rows, second, j);
+    const RowX2 p = weighted_rows<T>(YPDQ_W(1, 1), YPDQ_W(1, 2), YPDQ_W(1, 3),
+                                     load_rows(rows + 512, second + 512, j), nz);
+    float2 s = add2_rn(add2_rn(make_float2(0.0f, 0.0f), weighted_both<T>(YPDQ_W(0, 4), x.v[3], nz)),
+                       weighted_both<T>(YPDQ_W(0, 5), x.v[4], nz));
+    s = add_rows(s, p);
+    s = add_rows(s, weighted_rows<T>(YPDQ_W(2, 1), YPDQ_W(2, 2), YPDQ_W(2, 3),
+                                     load_rows(rows + 2 * 512, second + 2 * 512, j), nz));
+    s = add_rows(s, weighted_rows<T>(YPDQ_W(3, 1), YPDQ_W(3, 2), YPDQ_W(3, 3),
+                                     load_rows(rows + 3 * 512, second + 3 * 512, j), nz));
+    const RowX2 p4 = weighted_rows<T>(YPDQ_W(4, 1), YPDQ_W(4, 2), YPDQ_W(4, 3), x, nz);
+    const float2 done = add_rows(add_rows(make_float2(c.s, s.x), p4), p);
+    c.s = s.y;
+    return done;
+  }
+}
+
 // Separable compress (YPDQ_COMPRESS_SEPARABLE; not the reference's operation order). The
 // tent weights are W[di][dj] = c[di] c[dj] / 81 with c = (0, 1, 2, 3, 2, 1, 0) (the 128-bit
 // table also holds two subnormal residue taps, ~1e-40, which this form drops). So
@@ -271,6 +366,12 @@ __device__ __forceinline__ float compress_group(const Tin* rows, int j, bool las
     c.h3 = hsum(rows + 3 * 512, j);
   }
   return S * (1.0f / 81.0f);
+}
+template <typename Tin>
+__device__ __forceinline__ float2 compress_pair(const Tin* rows, int j, bool last, float,
+                                                HCarry& c) {
+  const float a = compress_group(rows, j, false, c);
+  return make_float2(a, compress_group(rows + 4 * 512, j, last, c));
 }
 
 // ---------------------------------------------------------------- epilogue
@@ -786,20 +887,24 @@ __global__ void __launch_bounds__(hash_threads<kDct>(), 2)
     // (value % 4) is known at compile time
 #pragma unroll 1
     for (int q = 0; q < kGroupsPerImage / 4; ++q) {
+      float2 pair = make_float2(0.0f, 0.0f);
 #pragma unroll
       for (int o = 0; o < 4; ++o) {
-        if (o % kGroups == 0 && !mbar_wait(&sm.full[slot], phase, abort_flag)) goto fail;
-        const Tin* rows =
-            reinterpret_cast<const Tin*>(sm.ring[slot] + (o % kGroups) * 4 * kRowBytes);
-        float b = compress_group(rows, jc, o == 3 && q == kGroupsPerImage / 4 - 1, carry);
-        if (o % kGroups == kGroups - 1) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.empty[slot]);
-          if (++slot == kNumStages) {
-            slot = 0;
-            phase ^= 1u;
+        if (o % 2 == 0) {
+          if (o % kGroups == 0 && !mbar_wait(&sm.full[slot], phase, abort_flag)) goto fail;
+          const Tin* rows =
+              reinterpret_cast<const Tin*>(sm.ring[slot] + (o % kGroups) * 4 * kRowBytes);
+          pair = compress_pair(rows, jc, o == 2 && q == kGroupsPerImage / 4 - 1, nz, carry);
+          if (o % kGroups == kGroups - 2) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.empty[slot]);
+            if (++slot == kNumStages) {
+              slot = 0;
+              phase ^= 1u;
+            }
           }
         }
+        float b = o % 2 == 0 ? pair.x : pair.y;
         const int i = 4 * q + o - 1;
         if (o == 0 && q == 0) b = 0.0f;  // there is no value -1
         if (buf1 && i >= 0) buf1[i * 128] = b;
@@ -912,8 +1017,8 @@ fail:
 // Bound by the latency of that sequence: of ~12,500 clk for one f32 image, ~2,800 until the
 // rows are there, ~2,000 compress (8 conflict-free 16-byte loads per value), ~500 for each of
 // the two exchanges, ~1,150 per DCT stage and ~4,200 epilogue (2,150 of them the gradient
-// sum). Back to back, one image: 8.5 us (hash_kernel 31 us for f32, 29 u8); RGB8 10.4 us (41);
-// 37 u8 images 14.5 us (29); 56 f32 images 27.3 us (31).
+// sum). Back to back, one image: 8.5 us (hash_kernel 31 us for f32, 27 u8); RGB8 10.4 us (39);
+// 37 u8 images 14.5 us (27); 56 f32 images 27.3 us (31).
 constexpr int kSplitCtas = 8;        // CTAs per image (the portable cluster size)
 constexpr int kSplitThreads = 512;
 constexpr int kSplitRows = 128 / kSplitCtas;           // compressed rows per CTA
@@ -1327,9 +1432,9 @@ static cudaError_t launch_split(const HashLaunch& p, cudaStream_t s) {
 
 // Largest batch that hash_split_kernel takes. Its time grows with the waves of clusters (16 or
 // more images at once), hash_kernel's is that of one image on a CTA up to 152 images (f32
-// 31-38 us, u8 29 us, RGB 41 us). Measured on both sides, split against persistent: f32
-// 27.3 / 31.1 us at 56 images and 32.0 / 31.4 at 64; u8 26.9 / 29.0 at 104 and 28.9 / 29.0 at
-// 112; RGB8 36.2 / 41.2 at 72 and 41.8 / 41.2 at 80; RGBA8 38.0 / 41.2 and 43.5 / 41.2.
+// 31-38 us, u8 27 us, RGB 39 us). Measured on both sides, split against persistent: f32
+// 27.3 / 31.1 us at 56 images and 32.0 / 31.4 at 64; u8 26.9 / 27.0 at 104 and 28.9 / 27.0 at
+// 112; RGB8 36.2 / 39.3 at 72 and 41.8 / 39.3 at 80; RGBA8 38.0 / 39.3 and 43.5 / 39.3.
 static int64_t split_max_images(int input_kind) {
   switch (input_kind) {
     case YPDQ_INPUT_F32: return 56;
