@@ -1017,12 +1017,15 @@ fail:
 // Bound by the latency of that sequence: of ~12,500 clk for one f32 image, ~2,800 until the
 // rows are there, ~2,000 compress (8 conflict-free 16-byte loads per value), ~500 for each of
 // the two exchanges, ~1,150 per DCT stage and ~4,200 epilogue (2,150 of them the gradient
-// sum). Back to back, one image: 8.5 us (hash_kernel 31 us for f32, 27 u8); RGB8 10.4 us (39);
-// 37 u8 images 14.5 us (27); 56 f32 images 27.3 us (31).
+// sum). Back to back, one image: 8.5 us (hash_kernel 31 us for f32, 27 u8); RGB8 9.6 us (39);
+// 37 u8 images 13.4 us (27); 56 f32 images 27.3 us (31).
 constexpr int kSplitCtas = 8;        // CTAs per image (the portable cluster size)
 constexpr int kSplitThreads = 512;
 constexpr int kSplitRows = 128 / kSplitCtas;           // compressed rows per CTA
 constexpr int kSplitInRows = 4 * kSplitRows + 2;       // input rows they read
+// compress_pair's last pair reads two rows more, for a start that nothing continues
+template <typename Tin>
+constexpr int kSplitPadRows = sizeof(Tin) == 1 ? 2 : 0;
 constexpr int kSplitCopies = (kSplitInRows + 15) / 16; // bulk copies of up to 16 rows
 
 constexpr int kSplitPitch = 132;  // floats per column of a stage's input (16-byte columns)
@@ -1225,15 +1228,26 @@ __global__ void __cluster_dims__(kSplitCtas, 1, 1) __launch_bounds__(kSplitThrea
   float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   const int i0 = kSplitRows * rank + 4 * g;
   if (j < 127) {
-    // the group before the first value starts it; group r + 1 finishes value r
+    // the group before the first value starts it; group r + 1 finishes value r (there is no
+    // value 127: what stands in its rows' place is summed and dropped)
     const Tin* st = reinterpret_cast<const Tin*>(rows + 16 * g * kRowBytes);
     TapSum carry;
     compress_group(st, j, false, carry);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (i0 + r < 127) {
-        b[r] = compress_group(st + 4 * (r + 1) * 512, j, r == 3 || i0 + r == 126, carry);
-        if (prm.buf1) prm.buf1[(n * 127 + i0 + r) * 128 + j] = b[r];
+    for (int r = 0; r < 4; r += 2) {
+      const Tin* next = st + 4 * (r + 1) * 512;
+      float2 pair;
+      if constexpr (sizeof(Tin) == 1) {  // 37 images 14.6 -> 13.4 us (RGB: 0.5 % slower)
+        pair = compress_pair(next, j, r == 2, prm.neg_zero, carry);
+      } else {
+        pair.x = compress_group(next, j, false, carry);
+        pair.y = compress_group(next + 4 * 512, j, r == 2, carry);
+      }
+      b[r] = pair.x;
+      b[r + 1] = i0 + r + 1 < 127 ? pair.y : 0.0f;
+      if (prm.buf1) {
+        prm.buf1[(n * 127 + i0 + r) * 128 + j] = pair.x;
+        if (i0 + r + 1 < 127) prm.buf1[(n * 127 + i0 + r + 1) * 128 + j] = pair.y;
       }
     }
   }
@@ -1416,7 +1430,8 @@ struct LaunchOne {
 
 template <typename Tin>
 static size_t split_smem_bytes() {
-  return kSplitRowsOffset + kSplitInRows * InputTraits<Tin>::kRowBytes + 128;  // + base alignment
+  return kSplitRowsOffset + (kSplitInRows + kSplitPadRows<Tin>) * InputTraits<Tin>::kRowBytes +
+         128;  // + base alignment
 }
 template <typename Tin>
 static cudaError_t set_split_smem() {
@@ -1433,8 +1448,8 @@ static cudaError_t launch_split(const HashLaunch& p, cudaStream_t s) {
 // Largest batch that hash_split_kernel takes. Its time grows with the waves of clusters (16 or
 // more images at once), hash_kernel's is that of one image on a CTA up to 152 images (f32
 // 31-38 us, u8 27 us, RGB 39 us). Measured on both sides, split against persistent: f32
-// 27.3 / 31.1 us at 56 images and 32.0 / 31.4 at 64; u8 26.9 / 27.0 at 104 and 28.9 / 27.0 at
-// 112; RGB8 36.2 / 39.3 at 72 and 41.8 / 39.3 at 80; RGBA8 38.0 / 39.3 and 43.5 / 39.3.
+// 27.3 / 31.1 us at 56 images and 32.0 / 31.4 at 64; u8 25.4 / 27.0 at 104 and 27.4 / 27.0 at
+// 112; RGB8 35.4 / 39.3 at 72 and 41.0 / 39.3 at 80; RGBA8 37.6 / 39.3 and 43.3 / 39.3.
 static int64_t split_max_images(int input_kind) {
   switch (input_kind) {
     case YPDQ_INPUT_F32: return 56;
