@@ -359,7 +359,7 @@ ypdq_status ypdq_hash_batch(ypdq_ctx* ctx, const void* d_images, int64_t n, int 
     const int64_t chunk = jarosz_chunk(n);
     if ((st = ensure_jarosz_scratch(ctx, chunk))) return st;
     CK(cudaStreamWaitEvent(s, ctx->jarosz_done, 0), "wait jarosz scratch");
-    CK(launch_hash_jarosz(p, ctx->jarosz_scratch, chunk, s), "jarosz launch");
+    CK(launch_hash_jarosz(p, ctx->jarosz_scratch, chunk, ctx->num_sms, s), "jarosz launch");
     CK(cudaEventRecord(ctx->jarosz_done, s), "record jarosz scratch");
     return YPDQ_OK;
   }
@@ -603,7 +603,7 @@ ypdq_status ypdq_screen_host(ypdq_ctx* ctx, ypdq_db* db, const void* h_images, i
     hp.dct = dct;
     hp.separable = sep;
     if (jarosz)
-      CK(launch_hash_jarosz(hp, ctx->jarosz_scratch, jchunk, s), "jarosz launch");
+      CK(launch_hash_jarosz(hp, ctx->jarosz_scratch, jchunk, ctx->num_sms, s), "jarosz launch");
     else
       CK(launch_hash(hp, ctx->num_sms, ctx->hash_ctas[hp.input_kind][dct][sep], s),
          "hash launch");

@@ -12,8 +12,8 @@
 //
 // Two ways through the filter, bit for bit the same:
 //   * jarosz_image_kernel, one CTA per image with every line's running sum kept on the chip
-//     (below): reads the image once and writes the PDQF. 1,500 u8 images 1,434 -> 413 us,
-//     456 f32 images 158 us.
+//     (below): reads the image once and writes the PDQF. 1,500 u8 images 1,434 -> 378 us,
+//     456 f32 images 150 us.
 //   * for fewer than 32 f32 or RGB images, where one CTA's walk over an image takes longer
 //     than short passes with a thread per line (one image 97 against 85 us f32, 106 against 88
 //     RGB8; at 32 images 101 against 110, 108 against 111): four launches through two f32
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(128) cols_dct_kernel(const float* __restrict__
 // p + 2 of the next pass.
 //
 // A step takes as long as its longest part: ~1,040 clk alone (u8: A 920, C 775, D 660, B 600),
-// ~1,400 with three CTAs per SM (shared memory), which keep the issue slots ~64 % busy. A
+// ~1,300 with three CTAs per SM (shared memory), which keep the issue slots ~64 % busy. A
 // running sum is two dependent additions per value, 8 clk, so 64 columns cannot take less
 // than ~510. The loads of each part come before its stores: the compiler may not move a
 // shared load over a shared store, and a load per quad of values made C take 1,900 clk. All
@@ -564,16 +564,42 @@ __device__ __forceinline__ void rows1_u8(const uint4 px, uint32_t& before, float
   }
 }
 
+// Where the four parts run, and when the CTAs of an SM start.
+//
+// A warp's scheduler is its hardware warp number modulo 4; a CTA's warps take consecutive ones
+// from a place that differs from CTA to CTA. Part A on one scheduler in all three CTAs makes
+// that scheduler the slowest, so the parts are turned by the CTA's place (hw_warp / 4), which
+// puts different parts on every scheduler: 456 u8 images 115 us, 1,500 378, 4,000 917 (turned
+// by the block index, which the hardware spreads over the SMs in an order of its own: 126, 410,
+// 962; the worst turn: 166, 394).
+//
+// CTAs that share an SM evenly also end together, and the SMs that end first take three of the
+// next images while others take none. So in the first of two or three waves the second and
+// third CTA start kStaggerNs and twice that later: 912 u8 images 225 us (231 without, 263 by
+// block index), 1,216 292 (315, 351), 912 RGB8 289 (306, 343); with more waves the ends drift
+// apart by themselves (2,000 images 500 us with, 477 without). With at most one image per SM
+// left over, none of this beats the turn by block index: 608 f32 images 246 us staggered, 237
+// by block; u8 185 both, 208 without a stagger.
+struct Parts {
+  bool by_block;           // parts turned by block index
+  uint32_t stagger_first;  // this many blocks start staggered
+};
+constexpr uint32_t kStaggerNs = 10000;
+
 template <int kKind>
 __global__ void __launch_bounds__(128, 3)
     jarosz_image_kernel(const uint8_t* __restrict__ in, float* __restrict__ pdqf,
-                        float* __restrict__ buf1, const int64_t* n_dev, int64_t i0, float nz) {
+                        float* __restrict__ buf1, const int64_t* n_dev, int64_t i0, float nz, Parts parts) {
   if (past_count(n_dev, i0, blockIdx.x)) return;  // the whole block: no barrier is split
   extern __shared__ __align__(16) uint8_t smem_raw[];
   ImageSmem<kKind>& sm = *reinterpret_cast<ImageSmem<kKind>*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // each part starts at another warp (scheduler) in each CTA
-  const int part = (warp + blockIdx.x) & 3;
+  // Each scheduler runs another part in each of its CTAs (see Parts).
+  __shared__ uint32_t hw_warp;
+  if (tid == 0) asm volatile("mov.u32 %0, %%warpid;" : "=r"(hw_warp));
+  __syncthreads();
+  const uint32_t slot = hw_warp >> 2;
+  const int part = (warp + (parts.by_block ? blockIdx.x : hw_warp + slot)) & 3;
   constexpr int kRowBytes = raw_row_bytes<kKind>();
   const uint8_t* img = in + blockIdx.x * kPlane * bytes_per_px<kKind>();
   auto fetch = [&](int t) {  // A: tile t's pixels into raw[t % 2], 16 bytes per lane and step
@@ -593,6 +619,10 @@ __global__ void __launch_bounds__(128, 3)
   for (int e = tid; e < 4 * 5 * 32; e += 128) (&sm.sample[0][0][0])[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int e = tid; e < kStrips * 2 * 32; e += 128) (&sm.col[0][0][0])[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (part == 1) fetch(0);
+  if (tid == 0 && blockIdx.x < parts.stagger_first) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < slot % 3 * kStaggerNs) __nanosleep(500);
+  }
   __syncthreads();
 
   Running<float> line = {};  // A: row sums of rows1; C: of rows2
@@ -755,8 +785,12 @@ cudaError_t image_init() {
 }
 template <int kKind>
 void launch_image(const uint8_t* in, float* pdqf, float* buf1, unsigned n, const int64_t* n_dev,
-                  int64_t i0, cudaStream_t s) {
-  jarosz_image_kernel<kKind><<<n, 128, sizeof(ImageSmem<kKind>), s>>>(in, pdqf, buf1, n_dev, i0, -0.0f);
+                  int64_t i0, int num_sms, cudaStream_t s) {
+  const unsigned sms = static_cast<unsigned>(num_sms), wave = 3 * sms;
+  const Parts parts = {n > wave && n <= wave + sms,
+                       n > wave + sms && n <= 3 * wave ? wave : 0u};
+  jarosz_image_kernel<kKind><<<n, 128, sizeof(ImageSmem<kKind>), s>>>(in, pdqf, buf1, n_dev, i0, -0.0f,
+                                                                       parts);
 }
 
 template <int kKind>
@@ -793,7 +827,8 @@ size_t jarosz_scratch_bytes(int64_t chunk) {
          static_cast<size_t>(chunk) * 256 * sizeof(float);
 }
 
-cudaError_t launch_hash_jarosz(const HashLaunch& p, void* scratch, int64_t chunk, cudaStream_t s) {
+cudaError_t launch_hash_jarosz(const HashLaunch& p, void* scratch, int64_t chunk, int num_sms,
+                               cudaStream_t s) {
   if (p.n <= 0) return cudaSuccess;
   static const size_t kBytesPerPixel[4] = {4, 1, 3, 4};
   if (p.input_kind < 0 || p.input_kind > 3) return cudaErrorInvalidValue;
@@ -809,10 +844,10 @@ cudaError_t launch_hash_jarosz(const HashLaunch& p, void* scratch, int64_t chunk
     if (p.n >= image_kernel_from(p.input_kind)) {
       const unsigned g = static_cast<unsigned>(m);
       switch (p.input_kind) {
-        case YPDQ_INPUT_F32: launch_image<YPDQ_INPUT_F32>(in, P, buf1, g, nd, i0, s); break;
-        case YPDQ_INPUT_U8: launch_image<YPDQ_INPUT_U8>(in, P, buf1, g, nd, i0, s); break;
-        case YPDQ_INPUT_RGB8: launch_image<YPDQ_INPUT_RGB8>(in, P, buf1, g, nd, i0, s); break;
-        default: launch_image<YPDQ_INPUT_RGBA8>(in, P, buf1, g, nd, i0, s); break;
+        case YPDQ_INPUT_F32: launch_image<YPDQ_INPUT_F32>(in, P, buf1, g, nd, i0, num_sms, s); break;
+        case YPDQ_INPUT_U8: launch_image<YPDQ_INPUT_U8>(in, P, buf1, g, nd, i0, num_sms, s); break;
+        case YPDQ_INPUT_RGB8: launch_image<YPDQ_INPUT_RGB8>(in, P, buf1, g, nd, i0, num_sms, s); break;
+        default: launch_image<YPDQ_INPUT_RGBA8>(in, P, buf1, g, nd, i0, num_sms, s); break;
       }
     } else {
       const dim3 grid(kN / 128, static_cast<unsigned>(m));

@@ -164,7 +164,7 @@ ypdq_status capture_bucket(ypdq_server* S, Slot& sl, const Bucket& b, cudaGraphE
   cudaError_t e = cudaMemcpyAsync(sl.d_hdr, sl.h_hdr, 16, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(&sl.d_hdr->count, 0, 16, s);
   if (e == cudaSuccess)
-    e = jarosz ? launch_hash_jarosz(hp, sl.d_jarosz, nb, s)
+    e = jarosz ? launch_hash_jarosz(hp, sl.d_jarosz, nb, S->ctx->num_sms, s)
                : launch_hash(hp, S->ctx->num_sms, S->ctx->hash_ctas[kind][hp.dct][hp.separable], s);
   if (e == cudaSuccess) e = launch_scan(sp, b.algo, S->ctx->num_sms, s);
   if (e == cudaSuccess)

@@ -308,7 +308,8 @@ cudaError_t launch_dihedrals(const DihedralLaunch& p, cudaStream_t s);
 // chunks of `chunk`, using `scratch` (jarosz_scratch_bytes(chunk) bytes).
 cudaError_t jarosz_init();
 size_t jarosz_scratch_bytes(int64_t chunk);
-cudaError_t launch_hash_jarosz(const HashLaunch& p, void* scratch, int64_t chunk, cudaStream_t s);
+cudaError_t launch_hash_jarosz(const HashLaunch& p, void* scratch, int64_t chunk, int num_sms,
+                               cudaStream_t s);
 
 // scan.cu
 cudaError_t scan_init();
