@@ -340,8 +340,8 @@ cudaError_t launch_scan(const ScanLaunch& p, int algo, int num_sms, cudaStream_t
 // ---------------------------------------------------------------- hit sorting
 //
 // By (index, query), the scalar matcher's visit order, through a second buffer: few hits by
-// counting for each the hits before it, more by a merge sort (tiles sorted in shared memory,
-// then passes that merge runs in pairs).
+// counting for each the hits before it; more by sorting tiles on the chip and merging these
+// runs, all at once while they are few, else in passes that merge them in pairs.
 
 // A hit as two words: the index, and query | distance << 32.
 struct Hit2 {
@@ -395,26 +395,69 @@ __global__ void __launch_bounds__(32 * kRankWarps)
   if (warp == 0 && i < n) store_hit(out, before[lane], x);
 }
 
-// The same in place for one block's worth of hits.
-constexpr int kSmallSort = 256;
-__global__ void __launch_bounds__(kSmallSort) rank_small_kernel(ypdq_hit* h, uint32_t n) {
-  __shared__ ulonglong2 all[kSmallSort];
+// Tile blockIdx.x of 256 hits sorted by ranks: each thread counts the hits of the tile before
+// its own (of equal ones the first first). in may be out.
+constexpr int kRankTile = 256;
+__global__ void __launch_bounds__(kRankTile)
+    rank_tiles_kernel(const ypdq_hit* in, ypdq_hit* out, uint64_t n) {
+  __shared__ ulonglong2 all[kRankTile];
+  const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kRankTile;
   const uint32_t i = threadIdx.x;
+  const uint32_t m = static_cast<uint32_t>(n - base < kRankTile ? n - base : kRankTile);
   Hit2 x{};
-  if (i < n) {
-    x = load_hit(h, i);
+  if (i < m) {
+    x = load_hit(in, base + i);
     all[i] = make_ulonglong2(x.k, (x.v << 32) | i);
   }
   __syncthreads();
-  if (i >= n) return;
+  if (i >= m) return;
   const uint64_t xs = (x.v << 32) | i;
   uint32_t c = 0;
 #pragma unroll 8
-  for (uint32_t j = 0; j < n; ++j) {
+  for (uint32_t j = 0; j < m; ++j) {
     const ulonglong2 y = all[j];
     c += is_before(y.x, y.y, x.k, xs);
   }
-  store_hit(h, c, x);
+  store_hit(out, base + c, x);
+}
+
+// All runs of w = 2^k sorted hits merged in one pass: a hit's place is its place in its run
+// plus, for every other run, how many of that run's hits come before it (of equal hits those
+// of the earlier run), k + 1 steps of a binary search. Block: 32 consecutive hits, one per
+// lane, whose searches stay close to each other; its warps share the runs.
+constexpr int kPlaceWarps = 16;
+__global__ void __launch_bounds__(32 * kPlaceWarps)
+    place_runs_kernel(const ypdq_hit* __restrict__ in, ypdq_hit* __restrict__ out, uint64_t n,
+                      uint32_t w) {
+  __shared__ uint32_t before[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t i = 32ull * blockIdx.x + lane;
+  if (warp == 0) before[lane] = 0;
+  __syncthreads();
+  const Hit2 x = load_hit(in, i < n ? i : n - 1);
+  const uint32_t runs = static_cast<uint32_t>((n + w - 1) / w);
+  const uint32_t own = static_cast<uint32_t>(32ull * blockIdx.x / w);
+  uint32_t c = 0;
+#pragma unroll 4
+  for (uint32_t r = warp; r < runs; r += kPlaceWarps) {
+    const ypdq_hit* run = in + static_cast<uint64_t>(r) * w;
+    const uint64_t left = n - static_cast<uint64_t>(r) * w;
+    const uint32_t m = left < w ? static_cast<uint32_t>(left) : w;
+    uint32_t at = 0;
+    if (r == own) {
+      at = static_cast<uint32_t>(i - static_cast<uint64_t>(own) * w);
+    } else {
+      for (uint32_t h = w; h > 0; h >>= 1) {
+        if (at + h > m) continue;
+        const Hit2 y = load_hit(run, at + h - 1);
+        if (r < own ? !less2(x, y) : less2(y, x)) at += h;
+      }
+    }
+    c += at;
+  }
+  atomicAdd(&before[lane], c);
+  __syncthreads();
+  if (warp == 0 && i < n) store_hit(out, before[lane], x);
 }
 
 constexpr int kSortItems = 8;  // hits per thread
@@ -667,19 +710,25 @@ cudaError_t sort_init() {
                               static_cast<int>(kSortSmem));
 }
 
-// Up to 256 hits: one block, in place. Up to 8,192: rank_hits_kernel (45 us there, event-timed
-// with its launches, against 64 for one tile and 60 for two tiles and a pass just above; at
-// 10,000 hits 67 against 60). Past that the merge sort. The bitonic sort that did all of this
-// before, in place with every step wider than 2,048 hits a launch of its own, took 23 us for
-// 100 hits (now 11), 39 for 1,000 (18), 85 for 8,192 (45), 107 for 10,000 (60), 200 for 100,000
-// (91) and 751 for 1.02 M (184); it stays for the case that the second buffer cannot be had.
-// Tiles of 4,096 hits: 2,048 and 8,192 take 190 and 177 us for 1.02 M but 63 and 73 for 10,000.
-constexpr uint64_t kRankMax = 8192;
+// Up to 256 hits: one block, in place. Past that, event-timed with their launches (us):
+//                     1,000  2,000  4,096  8,192  10,000  16,000  20,000  30,000  50,000  100,000
+//   rank_hits          18.6   20.8   30.0   44.7    67
+//   tiles 256, place   23.0   23.2   22.9   24.8    26.9    33.5    45.8    59.9   122.8
+//   tiles 1,024, place 30.6   33.9   33.3   33.7    33.8    35.9    39.5    43.0    64.1    145
+//   tiles 4,096, place 35.9   40.1   43.3   47.8    47.4    47.1    49.3    51.0    56.0     83
+//   tiles 4,096, pairs                              59.3    60.5    69.8    70.6    80.2     90
+// Placing costs hits x runs x log(run), which the pairs' passes overtake between 100,000 and
+// 150,000 hits (125 against 100 us). The bitonic sort that did all of this before, in place
+// with every step wider than 2,048 hits a launch of its own, took 23 us for 100 hits (now 11),
+// 39 for 1,000, 85 for 8,192, 107 for 10,000, 200 for 100,000 and 751 for 1.02 M (184); it
+// stays for the case that the second buffer cannot be had. For the pairs, tiles of 2,048 and
+// 8,192 hits take 190 and 177 us for 1.02 M, but 8,192 longer below it.
+constexpr uint64_t kRankMax = 2560, kPlaceMax256 = 16384, kPlaceMax1024 = 32768, kPlaceMax = 98304;
 
 cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cudaStream_t s) {
   if (n < 2) return cudaSuccess;
-  if (n <= static_cast<uint64_t>(kSmallSort)) {
-    rank_small_kernel<<<1, kSmallSort, 0, s>>>(hits, static_cast<uint32_t>(n));
+  if (n <= kRankTile) {
+    rank_tiles_kernel<<<1, kRankTile, 0, s>>>(hits, hits, n);
     return cudaGetLastError();
   }
   void* second = nullptr;
@@ -689,22 +738,32 @@ cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cud
   }
   ypdq_hit* const other = static_cast<ypdq_hit*>(second);
   cudaError_t e = cudaSuccess;
+  constexpr uint64_t kTile = kTileThreads * kSortItems;
+  const auto blocks = [n](uint64_t each) { return static_cast<unsigned>((n + each - 1) / each); };
+  const auto place = [&](uint32_t w) {
+    place_runs_kernel<<<blocks(32), 32 * kPlaceWarps, 0, s>>>(other, hits, n, w);
+  };
   if (n <= kRankMax) {
-    rank_hits_kernel<<<static_cast<unsigned>((n + 31) / 32), 32 * kRankWarps, 0, s>>>(
-        hits, other, static_cast<uint32_t>(n));
+    rank_hits_kernel<<<blocks(32), 32 * kRankWarps, 0, s>>>(hits, other, static_cast<uint32_t>(n));
     e = cudaMemcpyAsync(hits, other, n * sizeof(ypdq_hit), cudaMemcpyDeviceToDevice, s);
+  } else if (n <= kPlaceMax256) {
+    rank_tiles_kernel<<<blocks(kRankTile), kRankTile, 0, s>>>(hits, other, n);
+    place(kRankTile);
+  } else if (n <= kPlaceMax1024) {
+    sort_tiles_kernel<128><<<blocks(1024), 128, sizeof(Hit2) * padded(1024), s>>>(hits, other, n);
+    place(1024);
+  } else if (n <= kPlaceMax) {
+    sort_tiles_kernel<kTileThreads><<<blocks(kTile), kTileThreads, kSortSmem, s>>>(hits, other, n);
+    place(kTile);
   } else {
-    constexpr uint64_t kTile = kTileThreads * kSortItems;
     // the tiles go where an even number of passes from there ends in `hits`
     int passes = 0;
     for (uint64_t w = kTile; w < n; w <<= 1) ++passes;
     ypdq_hit* from = passes % 2 ? other : hits;
     ypdq_hit* to = passes % 2 ? hits : other;
-    sort_tiles_kernel<kTileThreads>
-        <<<static_cast<unsigned>((n + kTile - 1) / kTile), kTileThreads, kSortSmem, s>>>(hits, from, n);
+    sort_tiles_kernel<kTileThreads><<<blocks(kTile), kTileThreads, kSortSmem, s>>>(hits, from, n);
     for (uint64_t w = kTile; w < n; w <<= 1) {
-      merge_runs_kernel<<<static_cast<unsigned>((n + kMergeTile - 1) / kMergeTile), kMergeThreads, 0, s>>>(
-          from, to, n, w);
+      merge_runs_kernel<<<blocks(kMergeTile), kMergeThreads, 0, s>>>(from, to, n, w);
       ypdq_hit* t = from;
       from = to;
       to = t;
