@@ -129,7 +129,7 @@ typedef struct {
 
 /* Scan algorithms (all exact, all return the same hit set). */
 typedef enum {
-  YPDQ_SCAN_AUTO = 0,   /* pick by query count */
+  YPDQ_SCAN_AUTO = 0,   /* pick by query count, threshold and database size */
   YPDQ_SCAN_SIMT = 1,   /* XOR + popcount, one row per thread */
   YPDQ_SCAN_B1MMA = 2,  /* legacy binary MMA (mma.sync .b1 .xor.popc) */
   YPDQ_SCAN_TC = 3,     /* tcgen05 tensor cores on +-1 vectors: at threshold <= 36 block-scaled

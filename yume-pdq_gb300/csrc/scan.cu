@@ -287,15 +287,26 @@ cudaError_t scan_init() {
 // 9 SIMT queries at t <= 34 (10M rows: 0.072-0.078 ms against 0.066 ms for 8 SIMT queries
 // and 0.080 ms for 10), 6 at t = 35..36 (the SIMT side at three popcounts: 0.071 ms for 6,
 // 0.088 ms for 8), 24 at t <= 62 and 12 above (the FP8 passes, neither side pruned as far).
-int auto_scan_algo(uint32_t n_queries, uint32_t threshold) {
-  const uint32_t simt_max = threshold <= 34 ? 9 : threshold <= 36 ? 6 : threshold <= 62 ? 24 : 12;
+// A tensor-core launch takes ~9 us on any database (query expansion, a pipeline to fill), SIMT
+// ~6, so small databases move the line. SIMT against tensor cores without hits, t <= 34: 16
+// queries 16.9 / 18.0 us at 1 M rows, 25.9 / 26.2 at 2 M, 54.9 / 43.5 at 5 M (with 0.1 % of
+// the rows hits 17.2 / 23.1, 27.5 / 35.7, 58.0 / 69.1); 32 queries 9.3 / 10.6 at 100,000 rows,
+// 10.7 / 10.9 at 200,000, 15.2 / 12.8 at 500,000; 64 queries 11.0 / 9.1 at 50,000. At t = 35..36
+// 16 queries 9.7 / 12.7 at 200,000 rows, 14.3 / 16.3 at 500,000 (with hits; ~13 without).
+// Whole lookups from host queries to sorted hits gain more than the kernels, which change the
+// SM's shared-memory split back and forth: 16 queries against 100,000 rows 57.8 -> 47.7 us,
+// 1.5 M 81.5 -> 71.5; at t = 36 8 queries against 2 M rows 94 -> 81 (60.1 -> 57.5 without hits).
+int auto_scan_algo(uint32_t n_queries, uint32_t threshold, uint64_t n_rows) {
+  uint32_t simt_max = threshold <= 34 ? 9 : threshold <= 36 ? 6 : threshold <= 62 ? 24 : 12;
+  if (threshold <= 34 && n_rows <= 1500000) simt_max = n_rows <= 200000 ? 32 : 16;
+  if (threshold > 34 && threshold <= 36 && n_rows <= 2000000) simt_max = n_rows <= 200000 ? 16 : 8;
   return n_queries <= simt_max ? YPDQ_SCAN_SIMT : YPDQ_SCAN_TC;
 }
 
 cudaError_t launch_scan(const ScanLaunch& p, int algo, int num_sms, cudaStream_t s) {
   cudaError_t e = p.append ? cudaSuccess : cudaMemsetAsync(p.count, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess || p.n_rows == 0 || p.n_queries == 0) return e;
-  if (algo == YPDQ_SCAN_AUTO) algo = auto_scan_algo(p.n_queries, p.threshold);
+  if (algo == YPDQ_SCAN_AUTO) algo = auto_scan_algo(p.n_queries, p.threshold, p.n_rows);
   if (algo == YPDQ_SCAN_TC) return launch_scan_tc(p, num_sms, s);
   if (algo == YPDQ_SCAN_TC_FP4) {
     ScanLaunch q = p;

@@ -545,7 +545,7 @@ ypdq_status ypdq_server_create(ypdq_ctx* ctx, ypdq_db* db, const ypdq_server_con
   for (uint32_t b = 1; b <= cfg.max_step_images; b *= 2) {
     Bucket k;
     k.images = b;
-    k.algo = auto_scan_algo(8 * b, cfg.threshold);  // the ypdq_scan AUTO rule
+    k.algo = auto_scan_algo(8 * b, cfg.threshold, ~0ull);  // the AUTO rule of large databases
     S->buckets.push_back(k);
   }
   S->max_step = cfg.max_step_images;

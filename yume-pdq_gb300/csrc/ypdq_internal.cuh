@@ -314,9 +314,9 @@ cudaError_t launch_hash_jarosz(const HashLaunch& p, void* scratch, int64_t chunk
 // scan.cu
 cudaError_t scan_init();
 cudaError_t launch_scan(const ScanLaunch& p, int algo, int num_sms, cudaStream_t s);
-// the algorithm YPDQ_SCAN_AUTO runs for n_queries queries at threshold t
-int auto_scan_algo(uint32_t n_queries, uint32_t threshold);
-// past 8,192 hits a second buffer comes from `pool` (in stream order), if it can
+// the algorithm YPDQ_SCAN_AUTO runs for n_queries queries at threshold t on n_rows rows
+int auto_scan_algo(uint32_t n_queries, uint32_t threshold, uint64_t n_rows);
+// past 256 hits a second buffer comes from `pool` (in stream order), if it can
 cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cudaStream_t s);
 
 // scan_tc.cu
