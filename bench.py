@@ -255,11 +255,15 @@ def fp4_dense_burst(device=0, n=8192, reps=10):
         return None
 
 
-def scan_algo_used(algo, nq, threshold):
+def scan_algo_used(algo, nq, threshold, n_rows):
     """The algorithm ypdq_scan runs for YPDQ_SCAN_AUTO (mirrors auto_scan_algo in scan.cu)."""
     if algo == 0:
         simt_max = (9 if threshold <= 34 else 6 if threshold <= 36 else
                     24 if threshold <= 62 else 12)
+        if threshold <= 34 and n_rows <= 1500000:
+            simt_max = 32 if n_rows <= 200000 else 16
+        if 34 < threshold <= 36 and n_rows <= 2000000:
+            simt_max = 16 if n_rows <= 200000 else 8
         return 1 if nq <= simt_max else 3
     return algo
 
@@ -381,7 +385,7 @@ def large_db(yp, ctx, args, members=1000, trials=40, n_queries=1024):
     d_rows.free()
     d_hits.free()
     return {"workload": "%d clustered rows (%d centres x %d members, distance ~Binomial(%d, 1/2)) "
-                        "vs %d centre queries, tensor-core scan + bitonic sort of the hits"
+                        "vs %d centre queries, tensor-core scan + sort of the hits"
                         % (n, n_centres, members, trials, n_queries),
             "db_bytes": n * 32, "points": points}
 
@@ -402,7 +406,8 @@ def scan_sweep(yp, ctx, d_rows, n, d_hash, args, qs=(1, 8, 64, 256, 1024), reps=
     out = {"db_rows": n, "threshold": args.threshold, "hbm_peak_gbs": hbm_peak,
            "peak_source": peak_kind, "points": []}
     for q in qs:
-        pt = {"queries": q, "auto_algo": {1: "simt", 3: "tc"}[scan_algo_used(0, q, args.threshold)]}
+        pt = {"queries": q, "auto_algo": {1: "simt", 3: "tc"}[
+            scan_algo_used(0, q, args.threshold, n)]}
         for name, algo in (("simt", 1), ("tc", 3), ("tc_fp4", 4), ("auto", 0)):
             ms = []
             for rep in range(reps):
@@ -601,23 +606,28 @@ def run_ours(args):
     hbm_peak, bf16_peak, peak_kind = measured_peaks()
     hash_avg = statistics.mean(hash_ms)
     scan_avg = statistics.mean(scan_ms)
-    algo = scan_algo_used(args.algo, nq, args.threshold)
-    # the tensor-core form launch_scan_tc takes (mirrors it): at t <= 36 FP4 row triples up
-    # to 512 queries (launches of 128), FP4 query triples past that (passes of 720), or with
-    # YPDQ_SCAN_TC_FP8 FP8 query pairs past 256 (passes of 512) and single queries below;
-    # above t = 36 single queries (passes of 256)
+    algo = scan_algo_used(args.algo, nq, args.threshold, n)
+    # the tensor-core form launch_scan_tc takes (mirrors it): at t <= 36 FP4 query triples in
+    # passes of 720 and the queries left over as FP4 row triples (launches of 128) or one more
+    # pass, whichever it estimates faster; with YPDQ_SCAN_TC_FP8 FP8 query pairs past 256
+    # (passes of 512) and single queries below; above t = 36 single queries (passes of 256)
     low_t = args.threshold <= 36
+    whole, rest = divmod(nq, 720)
+    rows3_launches = (rest + 127) // 128
+    m_rows = n / 1e6
+    as_rows3 = rest > 0 and (rows3_launches * (8.0 + 7.0 * m_rows)
+                             < (1.4 if whole else 10.5) + 27.2 * m_rows)
     if low_t and args.algo != 5:
-        form = "rows3" if nq <= 512 else "triples"
+        form = "triples" if whole or not as_rows3 else "rows3"
     elif low_t:
         form = "pairs" if nq > 256 else "single"
     else:
         form = "single"
-    rows3_launches = (nq + 127) // 128
-    scan_launches = ((rows3_launches if form == "rows3" else 1) if algo in (3, 4, 5)
+    fp4_launches = (1 if whole or not as_rows3 else 0) + (rows3_launches if as_rows3 else 0)
+    scan_launches = ((fp4_launches if form in ("triples", "rows3") else 1) if algo in (3, 4, 5)
                      else (nq + 2047) // 2048)
     if scan_avg >= hash_avg and algo in (3, 4, 5):
-        # tensor-core scan, one launch per step: FP8 flops the MMAs execute per (row, query)
+        # tensor-core scan: flops the MMAs execute per (row, query)
         # pair, 2 * K: K = 128 at t <= 36 and 192 for passes of 256 queries at t <= 62 (the
         # prefix bound; mirrors launch_scan_tc), else 256. Peak: the dense FP8 burst measured
         # on this GPU in this run (else twice the measured bf16 burst, the nominal ratio).
@@ -628,7 +638,9 @@ def run_ours(args):
         triples = form in ("triples", "rows3")  # the FP4 forms
         pairs = form != "single"  # several queries (or rows) per accumulator column
         per_pass = {"triples": 720, "rows3": 128, "pairs": 512}.get(form, 256)
-        passes = (nq + per_pass - 1) // per_pass
+        passes = (nq + per_pass - 1) // per_pass  # database streams
+        if form == "triples" and as_rows3:
+            passes = whole + rows3_launches
         if triples:
             fp4 = fp4_dense_burst(local) if rank == 0 else None
             peak = fp4 if fp4 else 2 * fp8_dense_burst(local)
@@ -664,9 +676,9 @@ def run_ours(args):
                                        "4-pass launch over 10M rows (1.283 GB) per pass, scaled "
                                        "by this launch's passes and rows" if pairs else None),
                     "traffic_computed": passes * 32.0 * n + hits_per_step * 16.0,
-                    "traffic_note": "traffic_computed = 32 B x rows x %d query passes of %d + 16 B "
-                                    "per hit (the database streams once per pass), computed, not "
-                                    "a counter" % (passes, per_pass),
+                    "traffic_note": "traffic_computed = 32 B x rows x %d database streams (passes "
+                                    "of %d queries; left-over queries in launches of 128) + 16 B "
+                                    "per hit, computed, not a counter" % (passes, per_pass),
                     "mma_flop_note": "2 x %d FLOP per (row, query) pair: the K the MMAs execute "
                                      "per query" % k_bits,
                     "launch_ms": scan_avg / scan_launches, "launches_per_step": scan_launches,

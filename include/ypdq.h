@@ -87,9 +87,9 @@ typedef enum {
  * pdqhash-faithful kernel (src/kernel/mod.rs:690-820, src/kernel/ref.rs). Its compress runs
  * the full Jarosz filter (two box passes of window 3 along rows and columns of the whole
  * 512x512 image, running sums in f32) and samples it; its DCT sums each output in one
- * sequential accumulator. Bit-exact with that kernel for finite inputs. Slower (four passes
- * over the image through two f32 planes per image; the context keeps up to 4 GiB of
- * scratch for chunks of 2,048 images, and each server slot 2 MiB per image of its step).
+ * sequential accumulator. Bit-exact with that kernel for finite inputs. Slower (1,500 u8
+ * images 378 us). The context, and each server slot, keeps 62 MiB of scratch (two f32 planes for
+ * up to 31 images) and 1 KiB per image of a chunk of up to 16,384 (of a step).
  * Accepted by ypdq_hash_batch, ypdq_screen_host and ypdq_server_config.dct_precision.
  */
 #define YPDQ_COMPRESS_JAROSZ 0x200
@@ -133,10 +133,10 @@ typedef enum {
   YPDQ_SCAN_SIMT = 1,   /* XOR + popcount, one row per thread */
   YPDQ_SCAN_B1MMA = 2,  /* legacy binary MMA (mma.sync .b1 .xor.popc) */
   YPDQ_SCAN_TC = 3,     /* tcgen05 tensor cores on +-1 vectors: at threshold <= 36 block-scaled
-                           FP4 (e2m1) on the first 126 bits, up to 512 queries with three
-                           database rows per accumulator column (launches of 128 queries),
-                           past that three queries per column (passes of 720); above 36 FP8
-                           (dot = 256 - 2 d) */
+                           FP4 (e2m1) on the first 126 bits, three queries per accumulator
+                           column (passes of 720) and what is left with three database rows
+                           per column (launches of 128 queries) where that is faster; above
+                           36 FP8 (dot = 256 - 2 d) */
   YPDQ_SCAN_TC_FP4 = 4, /* the FP4 forms of YPDQ_SCAN_TC at threshold <= 36 (the same choice
                            between them); above that the same as YPDQ_SCAN_TC */
   YPDQ_SCAN_TC_FP8 = 5  /* tcgen05 with FP8 operands at every threshold: at threshold <= 36
