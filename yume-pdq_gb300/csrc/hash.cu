@@ -42,9 +42,10 @@
 //     slots: 375 us before the pairs; one slot after another: 1.3 us more for a single wave).
 // 4,096 u8 images: 552 -> 324 us (12.6 M images/s); 801 RGB8 images 262 -> 136 us; u8 with
 // the separable compress and the BF16x3 DCT, 1,024 images: 133 -> 72 us. No gain, measured: a
-// third CTA per SM (127 registers, copies and epilogue in one warp: 320 us against 324, single
-// waves 4 us longer, 801 RGB8 images 148 against 136), compress and DCT in warps of their own (388 against 375 us, none at
-// f32), a pair's DCT steps put beside the next pair's sums (the same times).
+// third CTA per SM (127 registers, copies and epilogue in one warp: 320 us against 324, but
+// single waves 4 us longer and 801 RGB8 images 148 against 136), compress and DCT in warps of
+// their own (388 against 375 us, none at f32), a pair's DCT steps put beside the next pair's
+// sums (the same times).
 #include <cuda_bf16.h>
 
 #include <cstring>
