@@ -449,6 +449,38 @@ __global__ void __launch_bounds__(kRankTile)
   store_hit(out, base + c, x);
 }
 
+// Up to 512 hits in place by one cluster of 8 CTAs: each keeps all hits in shared memory and
+// ranks 64 of them, eight warps to the same 32 hits; nobody writes before all have read.
+constexpr int kClusterSort = 512, kClusterSortCtas = 8, kClusterSortEach = 64;
+__global__ void __cluster_dims__(kClusterSortCtas, 1, 1) __launch_bounds__(512)
+    rank_cluster_kernel(ypdq_hit* h, uint32_t n) {
+  __shared__ ulonglong2 all[kClusterSort];
+  __shared__ uint32_t before[kClusterSortEach];
+  const uint32_t tid = threadIdx.x, own = tid % kClusterSortEach, part = tid / kClusterSortEach;
+  const uint32_t i = kClusterSortEach * blockIdx.x + own;
+  if (tid < n) {
+    const Hit2 y = load_hit(h, tid);
+    all[tid] = make_ulonglong2(y.k, (y.v << 32) | tid);
+  }
+  const Hit2 x = load_hit(h, min(i, n - 1));
+  if (tid < kClusterSortEach) before[tid] = 0;
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  const uint64_t xs = (x.v << 32) | i;
+  constexpr uint32_t kParts = 512 / kClusterSortEach;
+  const uint32_t each = (n + kParts - 1) / kParts, first = min(part * each, n), end = min(first + each, n);
+  uint32_t c = 0;
+#pragma unroll 8
+  for (uint32_t j = first; j < end; ++j) {
+    const ulonglong2 y = all[j];
+    c += is_before(y.x, y.y, x.k, xs);
+  }
+  atomicAdd(&before[own], c);
+  __syncthreads();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (tid < kClusterSortEach && i < n) store_hit(h, before[tid], x);
+}
+
 // All runs of w = 2^k sorted hits merged in one pass: a hit's place is its place in its run
 // plus, for every other run, how many of that run's hits come before it (of equal hits those
 // of the earlier run), k + 1 steps of a binary search. Block: 32 consecutive hits, one per
@@ -738,7 +770,10 @@ cudaError_t sort_init() {
                               static_cast<int>(kSortSmem));
 }
 
-// Up to 256 hits: one block, in place. Past that, event-timed with their launches (us):
+// Up to 256 hits: one block, in place. Up to 512 one cluster, in place too: 11.2 us for 512 hits,
+// event-timed with the launches, against 16.5 with rank_hits, a second buffer and a copy back; a
+// whole lookup with 500 hits 58.2 -> 52.7 us. (Up to 1,024 hits, 128 a CTA, it took 16.9 for 1,000
+// and lookups with 700 to 1,000 hits got 1-3 us longer.) Past that (us):
 //                     1,000  2,000  4,096  8,192  10,000  16,000  20,000  30,000  50,000  100,000
 //   rank_hits          18.6   20.8   30.0   44.7    67
 //   tiles 256, place   23.0   23.2   22.9   24.8    26.9    33.5    45.8    59.9   122.8
@@ -757,6 +792,10 @@ cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cud
   if (n < 2) return cudaSuccess;
   if (n <= kRankTile) {
     rank_tiles_kernel<<<1, kRankTile, 0, s>>>(hits, hits, n);
+    return cudaGetLastError();
+  }
+  if (n <= kClusterSort) {
+    rank_cluster_kernel<<<kClusterSortCtas, 512, 0, s>>>(hits, static_cast<uint32_t>(n));
     return cudaGetLastError();
   }
   void* second = nullptr;

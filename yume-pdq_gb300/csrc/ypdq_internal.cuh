@@ -316,7 +316,7 @@ cudaError_t scan_init();
 cudaError_t launch_scan(const ScanLaunch& p, int algo, int num_sms, cudaStream_t s);
 // the algorithm YPDQ_SCAN_AUTO runs for n_queries queries at threshold t on n_rows rows
 int auto_scan_algo(uint32_t n_queries, uint32_t threshold, uint64_t n_rows);
-// past 256 hits a second buffer comes from `pool` (in stream order), if it can
+// past 512 hits a second buffer comes from `pool` (in stream order), if it can
 cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cudaStream_t s);
 
 // scan_tc.cu
