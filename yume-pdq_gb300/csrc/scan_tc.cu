@@ -389,6 +389,7 @@ __device__ __noinline__ uint32_t push_candidates(uint32_t m, uint64_t row, uint3
   if (total <= kQueueHits) {
     for (uint32_t pos = count + before; m; m &= m - 1)
       queue->entry[pos++] = first + kStep * static_cast<uint32_t>(__ffs(static_cast<int>(m)) - 1);
+    __syncwarp();  // the callers' next tcgen05.ld is .sync.aligned: lanes leave the loop one by one
     return count + total;
   }
   // more than a queue's worth: a candidate of each lane at a time
@@ -404,6 +405,7 @@ __device__ __noinline__ uint32_t push_candidates(uint32_t m, uint64_t row, uint3
       count = 0;
     }
   }
+  __syncwarp();
   return count;
 }
 
