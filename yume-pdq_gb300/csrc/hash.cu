@@ -1272,13 +1272,22 @@ __global__ void __cluster_dims__(kSplitCtas, 1, 1) __launch_bounds__(kSplitThrea
   }
   cluster_arrive_relaxed();  // waited for at the end: no CTA leaves while another may write to it
   if (!ok && lane == 0) {
-    // data did not land in time: the outputs are not trustworthy. Give this warp's copy a
+    // data did not land in time (or another warp's did not): the outputs are not trustworthy.
+    // Everything still on its way into this CTA, copies and the other CTAs' stores alike, gets a
     // last bounded wait before the CTA may exit.
     *abort_flag = 1;
     atomicOr(prm.dev_err, kDevErrTimeout);
     const uint64_t t0 = globaltimer_ns();
-    while (!mbar_try_wait(&sm.full[g], 0) && globaltimer_ns() - t0 < kWaitLimitNs / 4) {
-    }
+    const auto landed = [t0](uint64_t* bar) {
+      while (!mbar_try_wait(bar, 0) && globaltimer_ns() - t0 < kWaitLimitNs / 4) {
+      }
+    };
+#pragma unroll 1
+    for (int c = 0; c < kSplitCopies; ++c)
+      if (row0 + 16 * c <= 510) landed(&sm.full[c]);
+    landed(&sm.dt_full);
+    landed(&sm.in_full[0]);
+    if (rank == 0) landed(&sm.in_full[1]);
   }
   if (rank == 0) {
     __syncthreads();
