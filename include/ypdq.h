@@ -271,7 +271,12 @@ ypdq_status ypdq_scan(ypdq_ctx *ctx, const uint8_t *d_rows, uint64_t n_rows,
                       ypdq_hit *d_hits, uint64_t capacity, uint64_t *d_count, int algo,
                       ypdq_stream_t stream);
 
-/* Sort n hits in place into the scalar matcher's visit order: index, then query. */
+/*
+ * Sort n hits in place into the scalar matcher's visit order: index, then query. Past 512 hits
+ * a second buffer of the same length is taken for the call, in stream order, from a pool of
+ * which the context keeps up to 64 MiB. Where it cannot be had, and on a stream under capture
+ * (the graph then holds kernels alone), a slower sort without it runs instead.
+ */
 ypdq_status ypdq_sort_hits(ypdq_ctx *ctx, ypdq_hit *d_hits, uint64_t n, ypdq_stream_t stream);
 
 /* ------------------------------------------------------------------ database */

@@ -784,8 +784,8 @@ cudaError_t sort_init() {
 // 150,000 hits (125 against 100 us). The bitonic sort that did all of this before, in place
 // with every step wider than 2,048 hits a launch of its own, took 23 us for 100 hits (now 11),
 // 39 for 1,000, 85 for 8,192, 107 for 10,000, 200 for 100,000 and 751 for 1.02 M (184); it
-// stays for the case that the second buffer cannot be had. For the pairs, tiles of 2,048 and
-// 8,192 hits take 190 and 177 us for 1.02 M, but 8,192 longer below it.
+// stays for a stream under capture and where the second buffer cannot be had. For the pairs,
+// tiles of 2,048 and 8,192 hits take 190 and 177 us for 1.02 M, but 8,192 longer below it.
 constexpr uint64_t kRankMax = 2560, kPlaceMax256 = 16384, kPlaceMax1024 = 32768, kPlaceMax = 98304;
 
 cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cudaStream_t s) {
@@ -798,8 +798,13 @@ cudaError_t launch_sort_hits(ypdq_hit* hits, uint64_t n, cudaMemPool_t pool, cud
     rank_cluster_kernel<<<kClusterSortCtas, 512, 0, s>>>(hits, static_cast<uint32_t>(n));
     return cudaGetLastError();
   }
+  // (Under capture the buffer would become allocation nodes of the graph, which then can be
+  // neither cloned nor a child graph nor instantiated twice.)
   void* second = nullptr;
-  if (!pool || cudaMallocFromPoolAsync(&second, n * sizeof(ypdq_hit), pool, s) != cudaSuccess) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (!pool || cudaStreamIsCapturing(s, &capture) != cudaSuccess ||
+      capture != cudaStreamCaptureStatusNone ||
+      cudaMallocFromPoolAsync(&second, n * sizeof(ypdq_hit), pool, s) != cudaSuccess) {
     cudaGetLastError();
     return launch_sort_in_place(hits, n, s);
   }
