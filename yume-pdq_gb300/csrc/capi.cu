@@ -244,20 +244,22 @@ ypdq_status ypdq_ctx_create(int device, ypdq_ctx** out) {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
     uint64_t keep = ypdq_ctx::kPoolKeep;
-    e = cudaMemPoolCreate(&ctx->pool, &props);
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    // (a device without pools has no fast hit sort, and nothing else misses one)
+    if (cudaMemPoolCreate(&ctx->pool, &props) == cudaSuccess) {
+      e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    } else {
+      ctx->pool = nullptr;
+      cudaGetLastError();
+    }
   }
   for (int i = 0; i < ypdq_ctx::kMaxChunks && e == cudaSuccess; ++i)
     e = cudaEventCreateWithFlags(&ctx->chunk_copied[i], cudaEventDisableTiming);
   if (e != cudaSuccess) {
-    if (ctx->h_err) cudaFreeHost(ctx->h_err);
-    delete ctx;
+    ypdq_ctx_destroy(ctx);
     return cuda_fail(e, "ypdq_ctx_create");
   }
   if (ctx->hash_ctas_f32 < 1 || ctx->hash_ctas_u8 < 1) {
-    cudaFreeHost(ctx->h_err);
-    cudaStreamDestroy(ctx->stream);
-    delete ctx;
+    ypdq_ctx_destroy(ctx);
     return fail(YPDQ_ERR_UNSUPPORTED, "hash kernel does not fit on this device");
   }
   *out = ctx;

@@ -32,7 +32,7 @@ struct ypdq_ctx {
   size_t jarosz_bytes = 0;
   cudaEvent_t jarosz_done = nullptr;  // recorded after the last work that used it
   // stream-ordered temporaries (the hit sort's second buffer); keeps at most kPoolKeep bytes
-  // between calls
+  // between calls; null if the device has no pools
   cudaMemPool_t pool = nullptr;
   static constexpr uint64_t kPoolKeep = 64ull << 20;
 };
