@@ -307,6 +307,8 @@ ypdq_status ypdq_db_save_file(ypdq_db *db, const char *path, uint64_t chunk_byte
  *   h_images     n * 512 * 512 f32 or u8 (pinned memory is fastest; any host memory works).
  *   h_hits       capacity entries; *n_hits gets the total (YPDQ_ERR_OVERFLOW if > capacity).
  *   h_hashes     n * 8 * 32 bytes, or NULL.  h_quality  n * 8 f32, or NULL.
+ * The context keeps page-locked memory for the results: the largest capacity seen, and up to
+ * 512 KiB of hashes and qualities (more go straight to the caller's memory).
  */
 ypdq_status ypdq_screen_host(ypdq_ctx *ctx, ypdq_db *db, const void *h_images, int64_t n,
                              int input_kind, int dct_precision, int semantics,

@@ -1,6 +1,4 @@
-"""ypdq_ctx_create on a machine that refuses one of its calls, with a stand-in for the CUDA
-runtime (tests/fake_cudart.c, no GPU): nothing created stays behind, and a device without memory
-pools is no reason to refuse."""
+"""Host paths against a stand-in for the CUDA runtime (tests/fake_cudart.c, no GPU)."""
 import os
 import shutil
 import subprocess
@@ -65,5 +63,45 @@ def run_with(fake, script, *args):
 
 
 def test_failed_creation_leaves_nothing(yp, fake_cudart):
+    """ypdq_ctx_create with one of its calls refused: nothing created stays behind, and a device
+    without memory pools is no reason to refuse."""
     yp._lib.load()
     run_with(fake_cudart, CREATE, yp._lib.LIB_PATH, str(yp._lib.ERR_UNSUPPORTED))
+
+
+SCREEN = r"""
+import ctypes, sys
+import numpy as np
+fake, lib = ctypes.CDLL(sys.argv[1]), ctypes.CDLL(sys.argv[2])
+fake.fake_most_pinned.restype = ctypes.c_size_t
+u64, vp = ctypes.c_uint64, ctypes.c_void_p
+lib.ypdq_screen_host.argtypes = [vp, vp, vp, ctypes.c_int64, ctypes.c_int, ctypes.c_int,
+                                 ctypes.c_int, ctypes.c_uint32, vp, u64, vp, vp, vp]
+lib.ypdq_db_wrap.argtypes = [vp, vp, u64, vp]
+ctx, db, total = vp(), vp(), u64(7)
+assert lib.ypdq_ctx_create(0, ctypes.byref(ctx)) == 0
+assert lib.ypdq_db_wrap(ctx, vp(1 << 20), 1000, ctypes.byref(db)) == 0
+capacity = 1000
+hits = np.zeros(capacity * 16, np.uint8)
+images = np.empty((8192, 512, 512), np.uint8)  # never touched
+for n in (1, 200, 1024, 2048, 8192):
+    fake.fake_reset(0)
+    for want_hashes, want_quality in ((1, 1), (1, 0), (0, 1), (0, 0)):
+        hashes, quality = np.full((n, 256), 0xAA, np.uint8), np.full((n, 8), 3, np.float32)
+        st = lib.ypdq_screen_host(ctx, db, images.ctypes.data, n, 1, 0, 0, 31, hits.ctypes.data,
+                                  capacity, ctypes.addressof(total),
+                                  hashes.ctypes.data if want_hashes else None,
+                                  quality.ctypes.data if want_quality else None)
+        assert st == 0 and total.value == 0, (st, total.value)
+        assert (hashes == (0 if want_hashes else 0xAA)).all()
+        assert (quality == (0 if want_quality else 3)).all()
+    assert fake.fake_most_pinned() <= 64 + 16 * capacity + (512 << 10), (n, fake.fake_most_pinned())
+print("ok")
+"""
+
+
+def test_screening_pins_no_memory_per_image(yp, fake_cudart):
+    """What ypdq_screen_host keeps page-locked grows with the hit capacity alone: the hashes and
+    qualities of many images go straight to the caller, and arrive in every combination."""
+    yp._lib.load()
+    run_with(fake_cudart, SCREEN, yp._lib.LIB_PATH)

@@ -624,11 +624,23 @@ ypdq_status ypdq_screen_host(ypdq_ctx* ctx, ypdq_db* db, const void* h_images, i
     CK(launch_scan(sp, YPDQ_SCAN_AUTO, ctx->num_sms, s), "scan launch");
   }
   if (jarosz && n > 0) CK(cudaEventRecord(ctx->jarosz_done, s), "record jarosz scratch");
-  // results come back through the page-locked staging buffer: [count][hits][hashes][quality]
+  // results come back through the page-locked staging buffer: [count][hits][hashes][quality];
+  // more hashes and qualities than kStageResults go straight to the caller's memory, so that
+  // what stays page-locked does not grow with the images
+  constexpr size_t kStageResults = 512 << 10;
+  const size_t hash_bytes = h_hashes ? 256 * n : 0, quality_bytes = h_quality ? 32 * n : 0;
+  const bool staged = hash_bytes + quality_bytes <= kStageResults;
   uint8_t* stage = nullptr;
   const size_t hits_at = 64, hashes_at = hits_at + sizeof(ypdq_hit) * capacity;
-  const size_t quality_at = hashes_at + (h_hashes ? 256 * n : 0);
-  if ((st = host_stage(ctx, quality_at + (h_quality ? 32 * n : 0), &stage))) return st;
+  const size_t quality_at = hashes_at + hash_bytes;
+  if ((st = host_stage(ctx, staged ? quality_at + quality_bytes : hashes_at, &stage))) return st;
+  const auto fetch_results = [&](void* hashes, void* quality) {
+    cudaError_t e = cudaSuccess;
+    if (hash_bytes) e = cudaMemcpyAsync(hashes, d_hash, hash_bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && quality_bytes)
+      e = cudaMemcpyAsync(quality, d_q, quality_bytes, cudaMemcpyDeviceToHost, s);
+    return e;
+  };
   CK(cudaMemcpyAsync(stage, d_cnt, sizeof(uint64_t), cudaMemcpyDeviceToHost, s), "D2H count");
   // the first hits come with the count: up to kHostSort are sorted here, without another round
   // trip (~15 us with the sort's launch; sorting 128 hits on a core takes ~4)
@@ -637,8 +649,7 @@ ypdq_status ypdq_screen_host(ypdq_ctx* ctx, ypdq_db* db, const void* h_images, i
   if (early > 0)
     CK(cudaMemcpyAsync(stage + hits_at, d_hits, early * sizeof(ypdq_hit), cudaMemcpyDeviceToHost, s),
        "D2H first hits");
-  if (h_hashes && n > 0) CK(cudaMemcpyAsync(stage + hashes_at, d_hash, 256 * n, cudaMemcpyDeviceToHost, s), "D2H hashes");
-  if (h_quality && n > 0) CK(cudaMemcpyAsync(stage + quality_at, d_q, 32 * n, cudaMemcpyDeviceToHost, s), "D2H quality");
+  if (staged) CK(fetch_results(stage + hashes_at, stage + quality_at), "D2H hashes and qualities");
   CK(cudaStreamSynchronize(s), "screen sync");
   uint64_t total = 0;
   memcpy(&total, stage, sizeof(total));
@@ -653,9 +664,13 @@ ypdq_status ypdq_screen_host(ypdq_ctx* ctx, ypdq_db* db, const void* h_images, i
     CK(launch_sort_hits(static_cast<ypdq_hit*>(d_hits), m, ctx->pool, s), "sort launch");
     CK(cudaMemcpyAsync(stage + hits_at, d_hits, m * sizeof(ypdq_hit), cudaMemcpyDeviceToHost, s), "D2H hits");
   }
-  if (h_hashes && n > 0) memcpy(h_hashes, stage + hashes_at, 256 * n);
-  if (h_quality && n > 0) memcpy(h_quality, stage + quality_at, 32 * n);
-  if (!all_here) CK(cudaStreamSynchronize(s), "screen sync");
+  if (!staged) {
+    CK(fetch_results(h_hashes, h_quality), "D2H hashes and qualities");
+  } else {
+    if (hash_bytes) memcpy(h_hashes, stage + hashes_at, hash_bytes);
+    if (quality_bytes) memcpy(h_quality, stage + quality_at, quality_bytes);
+  }
+  if (!all_here || !staged) CK(cudaStreamSynchronize(s), "screen sync");
   if (m > 0) memcpy(h_hits, stage + hits_at, m * sizeof(ypdq_hit));
   if ((st = read_device_errors(ctx))) return st;
   *n_hits = total;

@@ -24,8 +24,9 @@ struct ypdq_ctx {
   std::mutex mu;                  // guards the scratch buffers below
   void* scratch[8] = {};
   size_t scratch_bytes[8] = {};
-  // page-locked host staging of ypdq_screen_host's results (count, hits, hashes, qualities), so
-  // its device-to-host copies never take the driver's path for pageable memory
+  // page-locked host staging of ypdq_screen_host's results (count, hits, and up to 512 KiB of
+  // hashes and qualities), so that short device-to-host copies never take the driver's path for
+  // pageable memory; as long as the largest hit capacity seen asks for
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;
   void* jarosz_scratch = nullptr;  // YPDQ_COMPRESS_JAROSZ filter planes
