@@ -14,6 +14,8 @@ class Context:
 
     def __init__(self, device=0):
         self.lib = _lib.load()
+        self._spare = []  # (pointer, bytes) of returned buffers, see borrow
+        self._spare_lock = threading.Lock()
         h = ctypes.c_void_p()
         check(self.lib.ypdq_ctx_create(device, ctypes.byref(h)))
         self.handle = h
@@ -22,8 +24,6 @@ class Context:
         check(self.lib.ypdq_device_info(h, ctypes.byref(sms), ctypes.byref(ctas)))
         self.num_sms = sms.value
         self.hash_ctas_per_sm = ctas.value
-        self._spare = []  # (pointer, bytes) of returned buffers, see borrow
-        self._spare_lock = threading.Lock()
 
     def close(self):
         if self.handle:
