@@ -168,10 +168,15 @@ ChunkCost screen_chunk_cost(int input_kind, bool jarosz, uint64_t n_rows, uint32
   // the Jarosz filter: one CTA walks an image in 80-110 us however few the images, and three
   // CTAs share an SM
   if (jarosz) return {80.0, (input_kind == YPDQ_INPUT_U8 ? 0.28 : 0.37) + scan_us};
-  // hash_kernel runs one image per CTA, two CTAs per SM: a chunk of up to 304 images takes
-  // one image's time on a CTA, 304 x the per-image rate
-  const double hash_us = input_kind == YPDQ_INPUT_U8 ? 0.135 : input_kind == YPDQ_INPUT_F32 ? 0.18 : 0.28;
-  return {304.0 * hash_us, hash_us + scan_us};
+  // hash_kernel runs one image per CTA, two CTAs per SM: a chunk of up to 304 images takes one
+  // image's time on a CTA (27, 31 or 39 us), more the per-image rate; a chunk small enough for
+  // hash_split_kernel is priced like one wave too. 14 us are the launches and the scan's start.
+  // With the times of earlier kernels (55 us + 0.18 an image for f32, 85 + 0.28 for colour) chunks
+  // grew before the copies could keep up: 1,024 f32 images against 10 M rows 5.79 -> 5.51 ms, 600
+  // RGB8 2.86 -> 2.68, 2,048 RGB8 8.61 -> 8.29; 60,000 and 1 M rows the same to 1 %, but for 600
+  // to 2,048 images at t = 48, 1 M rows (f32 3.15 -> 3.08, 5.19 -> 5.29, 10.45 -> 10.33).
+  const bool u8 = input_kind == YPDQ_INPUT_U8, f32 = input_kind == YPDQ_INPUT_F32;
+  return {14.0 + (u8 ? 27.0 : f32 ? 31.0 : 39.0), (u8 ? 0.079 : f32 ? 0.16 : 0.15) + scan_us};
 }
 
 // The chunk plan of ypdq_screen_host (and ypdq_screen_plan).
