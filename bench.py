@@ -682,6 +682,9 @@ def run_ours(args):
                     "mma_flop_note": "2 x %d FLOP per (row, query) pair: the K the MMAs execute "
                                      "per query" % k_bits,
                     "launch_ms": scan_avg / scan_launches, "launches_per_step": scan_launches,
+                    "launch_note": ("mean of a launch of %d passes and %d launches of up to 128 "
+                                    "queries (scan_rows3_kernel)" % (whole, rows3_launches)
+                                    if form == "triples" and as_rows3 else None),
                     "mma_k_bits": k_bits,
                     "pairs_per_s": nq * n / (scan_avg / 1e3),
                     "db_stream_gbs": (n * 32 * passes) / (scan_avg / 1e3) / 1e9,

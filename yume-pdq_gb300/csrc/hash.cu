@@ -1000,8 +1000,8 @@ fail:
 //
 // hash_split_kernel: the FP32 hash of a small batch, one image per cluster of 8 CTAs.
 //
-// hash_kernel walks an image's 128 stages one after another on one CTA, ~40 us whatever the
-// batch, so a batch of fewer images than CTAs leaves most of the chip idle and waits for a
+// hash_kernel walks an image's 128 groups of rows one after another on one CTA, 27-39 us however
+// small the batch, so a batch of fewer images than CTAs leaves most of the chip idle and waits for a
 // latency chain. Here the image is cut by rows: CTA c of the cluster copies the 66 input
 // rows of compressed rows 16 c .. 16 c + 15 at once (five bulk copies, no ring), and the
 // chains that are serial by definition are cut along their independent directions:
@@ -1019,7 +1019,8 @@ fail:
 // rows are there, ~2,000 compress (8 conflict-free 16-byte loads per value), ~500 for each of
 // the two exchanges, ~1,150 per DCT stage and ~4,200 epilogue (2,150 of them the gradient
 // sum). Back to back, one image: 8.5 us (hash_kernel 31 us for f32, 27 u8); RGB8 9.6 us (39);
-// 37 u8 images 13.4 us (27); 56 f32 images 27.3 us (31).
+// 37 u8 images 13.4 us (27), or 14.2 when each call brings new ones, from HBM; 56 f32 images
+// 27.3 us (31).
 constexpr int kSplitCtas = 8;        // CTAs per image (the portable cluster size)
 constexpr int kSplitThreads = 512;
 constexpr int kSplitRows = 128 / kSplitCtas;           // compressed rows per CTA
@@ -1238,7 +1239,7 @@ __global__ void __cluster_dims__(kSplitCtas, 1, 1) __launch_bounds__(kSplitThrea
     for (int r = 0; r < 4; r += 2) {
       const Tin* next = st + 4 * (r + 1) * 512;
       float2 pair;
-      if constexpr (sizeof(Tin) == 1) {  // 37 images 14.6 -> 13.4 us (RGB: 0.5 % slower)
+      if constexpr (sizeof(Tin) == 1) {  // 37 images from L2 14.6 -> 13.4 us (RGB: 0.5 % slower)
         pair = compress_pair(next, j, r == 2, prm.neg_zero, carry);
       } else {
         pair.x = compress_group(next, j, false, carry);

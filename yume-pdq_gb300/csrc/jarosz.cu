@@ -579,7 +579,9 @@ __device__ __forceinline__ void rows1_u8(const uint4 px, uint32_t& before, float
 // block index), 1,216 292 (315, 351), 912 RGB8 289 (306, 343); with more waves the ends drift
 // apart by themselves (2,000 images 500 us with, 477 without). With at most one image per SM
 // left over, none of this beats the turn by block index: 608 f32 images 246 us staggered, 237
-// by block; u8 185 both, 208 without a stagger.
+// by block; u8 185 both, 208 without a stagger. (On 152 SMs. The delay is u8's best of 0, 10 and
+// 20 us, and the lines go by the number of images launched: a server step that replays a larger
+// bucket's graph with fewer keeps that bucket's rule.)
 struct Parts {
   bool by_block;           // parts turned by block index
   uint32_t stagger_first;  // this many blocks start staggered

@@ -284,9 +284,9 @@ cudaError_t scan_init() {
 // SIMT is HBM-bound up to a few queries; past that it is bound by its popcount and logic
 // pipes, at 2, 3 or 4 popcounts per pair depending on the threshold (the prefix bound in
 // scan_simt_kernel). A narrow tensor-core pass (at most 128 queries) costs about the time of
-// 9 SIMT queries at t <= 34 (10M rows: 0.072-0.078 ms against 0.066 ms for 8 SIMT queries
-// and 0.080 ms for 10), 6 at t = 35..36 (the SIMT side at three popcounts: 0.071 ms for 6,
-// 0.088 ms for 8), 24 at t <= 62 and 12 above (the FP8 passes, neither side pruned as far).
+// 9 SIMT queries at t <= 34 (10M rows without hits: 0.070-0.078 ms; SIMT 0.062 ms for 8
+// queries, 0.069 for 9, 0.074 for 10), 6 at t = 35..36 (the SIMT side at three popcounts: 0.068
+// ms for 6, 0.077 for 7), 24 at t <= 62 and 12 above (the FP8 passes, neither side pruned as far).
 // A tensor-core launch takes ~9 us on any database (query expansion, a pipeline to fill), SIMT
 // ~6, so small databases move the line. SIMT against tensor cores without hits, t <= 34: 16
 // queries 16.9 / 18.0 us at 1 M rows, 25.9 / 26.2 at 2 M, 54.9 / 43.5 at 5 M (with 0.1 % of

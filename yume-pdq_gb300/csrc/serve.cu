@@ -463,8 +463,9 @@ ypdq_status autotune(ypdq_server* S) {
     const uint32_t nq = 8 * b.images;
     if (nq <= 64) cand.push_back(Bucket{b.images, YPDQ_SCAN_SIMT, 0, 0, 0.0f, 0});
     // the launcher's choice: at t <= 36 queries as A with three database rows per column (FP4,
-    // one launch per 128 queries) up to 512 queries and FP4 triple passes of 720 past that;
-    // above t = 36 queries as A (FP8) up to 128 queries, then one query per column
+    // one launch per 128 queries) up to 512 queries (a step's count is on the device), past that
+    // FP4 triple passes of 720 and such launches for the rest where they cost less than one more
+    // pass; above t = 36 queries as A (FP8) up to 128 queries, then one query per column
     cand.push_back(Bucket{b.images, YPDQ_SCAN_TC, 0, 0, 0.0f, 0});
     const uint32_t nq64 = (nq + 63u) & ~63u;
     for (uint32_t nt = 64; nt <= 256; nt *= 2)

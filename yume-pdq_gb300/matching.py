@@ -20,7 +20,8 @@ class CudaVectorDatabase(core.Database):
 
 class CudaMatcher:
     """PDQMatcher over a CudaVectorDatabase with a fixed threshold. Calls borrow their device
-    buffers from the context, so threads can share a matcher."""
+    buffers from the context, so threads can share a matcher. (The word in which a scan reports
+    that it gave up waiting is the context's: one of the threads that wait on it gets the error.)"""
 
     InputDimension = 32
     NoFalseNegative = True
