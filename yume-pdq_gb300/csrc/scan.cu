@@ -287,15 +287,18 @@ cudaError_t scan_init() {
 // 9 SIMT queries at t <= 34 (10M rows without hits: 0.070-0.078 ms; SIMT 0.062 ms for 8
 // queries, 0.069 for 9, 0.074 for 10), 6 at t = 35..36 (the SIMT side at three popcounts: 0.068
 // ms for 6, 0.077 for 7), 24 at t <= 62 and 12 above (the FP8 passes, neither side pruned as far).
-// A tensor-core launch takes ~9 us on any database (query expansion, a pipeline to fill), SIMT
-// ~6, so small databases move the line. SIMT against tensor cores without hits, t <= 34: 16
-// queries 16.9 / 18.0 us at 1 M rows, 25.9 / 26.2 at 2 M, 54.9 / 43.5 at 5 M (with 0.1 % of
-// the rows hits 17.2 / 23.1, 27.5 / 35.7, 58.0 / 69.1); 32 queries 9.3 / 10.6 at 100,000 rows,
-// 10.7 / 10.9 at 200,000, 15.2 / 12.8 at 500,000; 64 queries 11.0 / 9.1 at 50,000. At t = 35..36
-// 16 queries 9.7 / 12.7 at 200,000 rows, 14.3 / 16.3 at 500,000 (with hits; ~13 without).
-// Whole lookups from host queries to sorted hits gain more than the kernels, which change the
-// SM's shared-memory split back and forth: 16 queries against 100,000 rows 57.8 -> 47.7 us,
-// 1.5 M 81.5 -> 71.5; at t = 36 8 queries against 2 M rows 94 -> 81 (60.1 -> 57.5 without hits).
+// A tensor-core launch takes ~8 us on any database (query expansion, a pipeline to fill), SIMT
+// ~6, and a few hits cost the tensor cores 2-5 us more, SIMT next to nothing, so small databases
+// move the line. SIMT against tensor cores, t <= 34, 16 queries: 8.2 / 8.4 us at 200,000 rows,
+// 10.5 / 10.3 at 500,000, 16.6 / 14.2 at 1 M, 20.8 / 16.6 at 1.5 M where nothing hits; 15.4 / 17.6
+// at 1 M and 21.1 / 21.3 at 1.5 M with some tens of hits; 16.9 / 22.9 and 23.1 / 29.2 with 0.1 % of
+// the rows. 32 queries 8.5 / 8.1 at 100,000 rows and 10.3 / 8.4 at 200,000 without a hit, 9.1 / 11.3
+// and 11.1 / 12.6 with 0.1 %. At t = 35..36 16 queries 8.5 / 8.9 at 200,000 rows (9.2 / 12.9 with
+// hits), 8 queries 21.6 / 21.6 at 2 M (22.1 / 35.5).
+// Whole lookups from host queries to sorted hits, with 0.1 %: 16 queries against 100,000 rows
+// 57.8 -> 47.7 us, 1.5 M 81.5 -> 71.5; at t = 36 8 queries against 2 M rows 94 -> 81. Where nothing
+// hits, the line costs up to 4 us of 31-44: 16 queries 31.1 / 30.6 at 200,000 rows, 43.8 / 40.6 at
+// 1.5 M, 32 queries 34.8 / 30.7 at 200,000.
 int auto_scan_algo(uint32_t n_queries, uint32_t threshold, uint64_t n_rows) {
   uint32_t simt_max = threshold <= 34 ? 9 : threshold <= 36 ? 6 : threshold <= 62 ? 24 : 12;
   if (threshold <= 34 && n_rows <= 1500000) simt_max = n_rows <= 200000 ? 32 : 16;
